@@ -539,6 +539,7 @@ int gx_ctx_destroy(gx_ctx *ctx)
   for (void *p : c->owned) cudaFree(p);
   if (c->host_buf) cudaFree(c->host_buf);
   if (c->host_stream) cudaStreamDestroy(c->host_stream);
+  if (c->flags) cudaFreeHost(c->flags);
   delete c;
   return GX_OK;
 }

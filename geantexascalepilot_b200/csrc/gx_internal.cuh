@@ -5,6 +5,7 @@
 #include "gx_csg.cuh"
 #include "gx_device.cuh"
 
+#include <mutex>
 #include <vector>
 
 namespace gx {
@@ -28,6 +29,13 @@ struct Ctx {
   double *csg_planes = nullptr;
   int csg_n = 0, csg_nscore = 0;
   int csg_solids = 0; // the solid kinds in the tree (bit k: kind k)
+  // error words of the calls that report one at once (gx_interact): host
+  // memory the kernels can write, one word per call in flight (a set bit of
+  // flags_used), so that such a call allocates and copies nothing
+  static constexpr int kFlags = 64;
+  std::mutex flags_mu;
+  int *flags = nullptr;
+  uint64_t flags_used = 0;
   double *stage_scratch = nullptr; // escaped energy of the stage calls (gx_along_step)
   // gx_transport_run_host: its stream and device staging buffer, kept across calls
   cudaStream_t host_stream = nullptr;

@@ -63,8 +63,10 @@ __global__ void __launch_bounds__(kBlock) k_rng_substreams(const uint64_t *__res
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= n) return;
   uint32_t v1[3] = {base[0], base[1], base[2]}, v2[3] = {base[3], base[4], base[5]};
-  matvec3(near + threadIdx.x, kBlock, v1, 0);
-  matvec3(near + 9 * kBlock + threadIdx.x, kBlock, v2, 1);
+  if (threadIdx.x != 0) {
+    matvec3(near + threadIdx.x, kBlock, v1, 0);
+    matvec3(near + 9 * kBlock + threadIdx.x, kBlock, v2, 1);
+  }
   out[0LL * n + i] = v1[0];
   out[1LL * n + i] = v1[1];
   out[2LL * n + i] = v1[2];
@@ -240,7 +242,7 @@ __global__ void k_interact(const Data *__restrict__ d, InterArgs a)
     a.sec_E[2 * i + s] = has ? io.sec_E[s] : 0.0;
     for (int k = 0; k < 3; ++k) a.sec_dir[6 * i + 3 * s + k] = has ? io.sec_dir[s][k] : 0.0;
   }
-  if (err) atomicOr(a.err, err);
+  if (err) atomicOr_system(a.err, err);
 }
 
 __global__ void k_field_value(const Data *__restrict__ d, int n, const double *__restrict__ pos,
@@ -336,6 +338,49 @@ static int check_launch(const char *what)
 } // namespace gx
 
 using namespace gx;
+
+// An error word of the context for one call, zeroed; when all are in use, one
+// of the call's own.  (A device word from the stream-ordered allocator cost a
+// call of 200003 interactions 0.5 ms: its pool returned the memory at every
+// synchronisation and mapped it again at the next call.)
+struct ErrorWord {
+  Ctx *C;
+  int slot = -1;
+  int *word = nullptr;
+  cudaError_t err = cudaSuccess;
+  explicit ErrorWord(Ctx *c) : C(c)
+  {
+    std::lock_guard<std::mutex> lk(C->flags_mu);
+    if (!C->flags) {
+      err = cudaHostAlloc((void **)&C->flags, Ctx::kFlags * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+      if (err != cudaSuccess) {
+        C->flags = nullptr;
+        return;
+      }
+    }
+    for (int k = 0; k < Ctx::kFlags && slot < 0; ++k)
+      if (!(C->flags_used >> k & 1)) slot = k;
+    if (slot >= 0) {
+      C->flags_used |= 1ULL << slot;
+      word = C->flags + slot;
+    } else if ((err = cudaHostAlloc((void **)&word, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped)) !=
+               cudaSuccess) {
+      word = nullptr;
+    }
+    if (word) *word = 0;
+  }
+  ErrorWord(const ErrorWord &) = delete;
+  ErrorWord &operator=(const ErrorWord &) = delete;
+  ~ErrorWord()
+  {
+    if (slot >= 0) {
+      std::lock_guard<std::mutex> lk(C->flags_mu);
+      C->flags_used &= ~(1ULL << slot);
+    } else if (word) {
+      cudaFreeHost(word);
+    }
+  }
+};
 
 #define GX_CTX(c)                                                                                                    \
   if (!(c)) return set_error(GX_ERR_ARG, "%s: null context", __func__);                                            \
@@ -461,20 +506,15 @@ int gx_interact(gx_ctx *ctx, int model, const gx_model_params *p, int n, uint32_
   a.sec_type = d_sec_type;
   a.sec_E = d_sec_E;
   a.sec_dir = d_sec_dir;
-  int *derr = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&derr, sizeof(int), stream_of(s));
-  if (e != cudaSuccess) return cuda_error(e, "gx_interact scratch");
-  cudaMemsetAsync(derr, 0, sizeof(int), stream_of(s));
-  a.err = derr;
+  ErrorWord word(C);
+  if (word.err != cudaSuccess) return cuda_error(word.err, "gx_interact error word");
+  a.err = word.word;
   k_interact<<<grid_for(n), kBlock, 0, stream_of(s)>>>(C->dev, a);
   int rc = check_launch("k_interact");
-  int herr = 0;
-  cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, stream_of(s));
-  cudaFreeAsync(derr, stream_of(s));
-  e = cudaStreamSynchronize(stream_of(s));
+  const cudaError_t e = cudaStreamSynchronize(stream_of(s));
   if (rc) return rc;
   if (e != cudaSuccess) return cuda_error(e, "gx_interact");
-  if (herr) return set_error(GX_ERR_ITERCAP, "gx_interact: a rejection loop hit its iteration cap");
+  if (*(volatile int *)word.word) return set_error(GX_ERR_ITERCAP, "gx_interact: a rejection loop hit its iteration cap");
   return GX_OK;
 }
 
