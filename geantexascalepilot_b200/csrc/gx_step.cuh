@@ -1,6 +1,5 @@
-// gx_step.cuh -- one step of a track, shared by the transport engines
-// (gx_transport.cu, gx_resident.cuh): the SoA track record, the layered
-// calorimeter's navigation, cross sections, multiple scattering, the phases of
+// gx_step.cuh -- one step of a track, for the transport engine
+// (gx_transport.cu): the track record, the layered calorimeter's navigation, cross sections, multiple scattering, the phases of
 // a step, the interaction models' dispatch, and the tallies of a block.
 #pragma once
 
@@ -18,9 +17,10 @@ namespace parity {
 // A track record: 96 bytes (128 in FP64), moved as 16-byte words.  One record
 // is three (four) whole sectors wherever it goes, whether one lane of a warp
 // writes or all, and takes 6 (8) memory instructions from one address.  As a
-// plane per member (23 words from 15 addresses, whose pointers had to be loaded
-// for each record) the e- kernel, whose tracks take 1.4 steps between a load
-// and a store, spent more on its records than on their steps' tables.
+// plane per member (23 words from 15 addresses, whose pointers were loaded for
+// each record, each written lane a sector per plane) 20000 10 GeV showers took
+// 172.0 ms, with these records and relocate() without its division 156.1 ms:
+// an e- takes 1.4 steps between a load and a store.
 // r0: multiple scattering: range scale of the step limit in the current volume
 // (<= 0: unset); rs: MRG32k3a state.
 template <class R> struct alignas(16) Rec {
@@ -1368,22 +1368,28 @@ __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 __device__ __forceinline__ unsigned lanemask_lt() { return (1u << lane_id()) - 1u; }
 
-// Reserve `cnt` consecutive slots per lane (0 <= cnt <= 3: a survivor and up
-// to two secondaries) in counter *ctr: one atomic per warp, returns this
-// lane's first slot.  The lanes' counts go in as two ballots (their bits 0
-// and 1), so the exclusive prefix is two popcounts instead of a shuffle scan;
-// the slots are those of the scan, in lane order.
-__device__ __forceinline__ long long warp_reserve(unsigned long long *ctr, int cnt)
+// Reserve cnt[q] consecutive slots per lane (0 to 3: a survivor and up to two
+// secondaries) in each of the counters ctr[q], q < nq <= 3: next[q] becomes this
+// lane's first slot.  The lanes' counts go in as two ballots per counter (their
+// bits 0 and 1), so the exclusive prefix is two popcounts; lane q adds to
+// counter q, so the three additions are in flight together instead of each
+// waiting for the one before.
+__device__ __forceinline__ void warp_reserve3(unsigned long long *ctr, int nq, const int cnt[3], long long next[3])
 {
-  const unsigned b0 = __ballot_sync(0xffffffffu, cnt & 1), b1 = __ballot_sync(0xffffffffu, cnt & 2);
-  const int total = __popc(b0) + 2 * __popc(b1);
-  if (total == 0) return 0;
-  const unsigned lt = lanemask_lt();
-  const int leader = __ffs(b0 | b1) - 1;
+  unsigned b0[3], b1[3];
+  int mine = 0;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    b0[q] = __ballot_sync(0xffffffffu, cnt[q] & 1);
+    b1[q] = __ballot_sync(0xffffffffu, cnt[q] & 2);
+    if ((int)lane_id() == q && q < nq) mine = __popc(b0[q]) + 2 * __popc(b1[q]);
+  }
   unsigned long long base = 0;
-  if ((int)lane_id() == leader) base = atomicAdd(ctr, (unsigned long long)total);
-  base = __shfl_sync(0xffffffffu, base, leader);
-  return (long long)base + __popc(b0 & lt) + 2 * __popc(b1 & lt);
+  if (mine) base = atomicAdd(ctr + lane_id(), (unsigned long long)mine);
+  const unsigned lt = lanemask_lt();
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    next[q] = (long long)__shfl_sync(0xffffffffu, base, q) + __popc(b0[q] & lt) + 2 * __popc(b1[q] & lt);
 }
 
 // Write a track to store q, or to q's overflow stack when the store is full.
@@ -1406,6 +1412,11 @@ template <class R> __device__ __forceinline__ void put_track(const Args<R> &a, i
 }
 
 // ----------------------------------------------------------------- kernels
+// Event row 0 of the tally lives in shared memory when it fits.  (The bins in
+// several copies, so that fewer lanes of a warp meet on one, were no gain: 8
+// copies of 100 bins 135.7 against 134.2 ms for 20000 showers.)
+constexpr int kTallyDoubles = 768;
+
 // Shared-memory tally and block statistics of one step kernel.
 __device__ __forceinline__ void tally_begin(Local &L, const Geom &g, double *edep, double *sm_edep,
                                             unsigned long long *sm_stat, double *sm_esc, int *sm_err)
@@ -1415,8 +1426,7 @@ __device__ __forceinline__ void tally_begin(Local &L, const Geom &g, double *ede
   L.g_edep = edep;
   L.sm_edep = sm_edep;
   L.sm_esc = sm_esc;
-  // event row 0 of the tally lives in shared memory when it fits in 6 KB
-  L.sm_bins = (g.nvol <= 768) ? g.nvol : 0;
+  L.sm_bins = (g.nvol <= kTallyDoubles) ? g.nvol : 0;
   for (int k = threadIdx.x; k < L.sm_bins; k += blockDim.x) sm_edep[k] = 0.0;
   for (int k = threadIdx.x; k < kNStat; k += blockDim.x) sm_stat[k] = 0;
   if (threadIdx.x == 0) {
@@ -1430,6 +1440,17 @@ __device__ __forceinline__ void tally_begin(Local &L, const Geom &g, double *ede
   for (int k = 0; k < kNStat; ++k) L.st[k] = 0;
 }
 
+// The sum of v over the lanes that are here, added to *ctr by one of them: a
+// 64-bit (or FP64) addition in shared memory is a compare-and-swap loop, and
+// every thread's own at the end of a block kept it there longer than an
+// interaction's sampling did.
+__device__ __forceinline__ void add_warp(unsigned long long *ctr, unsigned int v)
+{
+  const unsigned m = __activemask();
+  const unsigned sum = __reduce_add_sync(m, v);
+  if ((int)lane_id() == __ffs(m) - 1) atomicAdd(ctr, (unsigned long long)sum);
+}
+
 // steps_slot >= 0: the stat that also receives this kernel's step count
 __device__ __forceinline__ void tally_end(Local &L, Ctl *ctl, double *edep, double *sm_edep,
                                           unsigned long long *sm_stat, double *sm_esc, int *sm_err,
@@ -1437,9 +1458,13 @@ __device__ __forceinline__ void tally_end(Local &L, Ctl *ctl, double *edep, doub
 {
 #pragma unroll
   for (int k = 0; k < kNStat; ++k)
-    if (L.st[k]) atomicAdd(&sm_stat[k], (unsigned long long)L.st[k]);
-  if (steps_slot >= 0 && L.st[S_STEPS]) atomicAdd(&sm_stat[steps_slot], (unsigned long long)L.st[S_STEPS]);
-  if (L.retired != 0.0) atomicAdd(&sm_esc[1], L.retired);
+    if (L.st[k]) add_warp(&sm_stat[k], L.st[k]);
+  if (steps_slot >= 0 && L.st[S_STEPS]) add_warp(&sm_stat[steps_slot], L.st[S_STEPS]);
+  __syncwarp();
+  double retired = L.retired;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) retired += __shfl_xor_sync(0xffffffffu, retired, o);
+  if (lane_id() == 0 && retired != 0.0) atomicAdd(&sm_esc[1], retired);
   if (L.err) atomicOr(sm_err, L.err);
   __syncthreads();
   for (int k = threadIdx.x; k < L.sm_bins; k += blockDim.x)

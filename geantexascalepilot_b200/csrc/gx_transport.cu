@@ -1,8 +1,8 @@
 // gx_transport.cu -- the transport engine: every alive track takes one step
 // per iteration, in FP64 or FP32-mixed arithmetic.
 //
-// Layout in HBM: per particle type (gamma, e-, e+) two SoA track stores of
-// `capacity` slots (current / next) and one overflow stack.  A step kernel
+// Layout in HBM: per particle type (gamma, e-, e+) two track stores of
+// `capacity` records (current / next) and one overflow stack.  A step kernel
 // reads the current store of its type, runs one OneStep per track and writes
 // the survivor and its secondaries to the next stores through warp-aggregated
 // slot reservations (prefix sums over the warp, one atomic per warp and type),
@@ -59,9 +59,7 @@ __device__ __forceinline__ void emit_tracks(const Args<R> &a, Ctl *ctl, int par,
   for (int k = 0; k < 2; ++k)
     if (k < sec.n) take3(cnt, mixed ? 0 : sec.type[k], 1);
   long long next[3];
-#pragma unroll
-  for (int q = 0; q < 3; ++q)
-    next[q] = (q < a.nstores) ? warp_reserve((unsigned long long *)&ctl->count[par ^ 1][q], cnt[q]) : 0;
+  warp_reserve3((unsigned long long *)ctl->count[par ^ 1], a.nstores, cnt, next);
   if (!active) return;
   Mrg rng = t.rng();
 #pragma unroll
@@ -163,20 +161,6 @@ template <class R, int PT, int K> __global__ void __launch_bounds__(256, 2) k_st
 template <class R> constexpr int kMinBlocks = sizeof(R) == 8 ? 2 : 0; // 0: no minimum
 template <class R, int K> constexpr int kMaxRegs = sizeof(R) == 8 ? 128 : (K == 0 ? 96 : 255);
 
-// One slot per flagged lane in counter *ctr (ballot and popcount, one atomic
-// per warp when any lane is flagged); returns this lane's slot, 0 for lanes
-// not flagged.  Every lane of the warp calls it.
-__device__ __forceinline__ long long warp_take1(unsigned long long *ctr, bool flag)
-{
-  const unsigned m = __ballot_sync(0xffffffffu, flag);
-  if (!m) return 0;
-  const int leader = __ffs(m) - 1;
-  unsigned long long base = 0;
-  if ((int)lane_id() == leader) base = atomicAdd(ctr, (unsigned long long)__popc(m));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  return flag ? (long long)base + __popc(m & lanemask_lt()) : 0;
-}
-
 // Timeline tracing (the library built with GX_TIMELINE, a separate build of
 // this file): per iteration and step kernel, the global timer when the first
 // block of the kernel starts and when the last one ends, so that a run shows
@@ -251,6 +235,7 @@ template <class R, int PT, int K> __device__ __forceinline__ void transport_body
   bool have = false, more = true; // `more` is warp-uniform: the work counter is not exhausted
   bool infield = false;           // in the middle of a step (helix sub-steps)
   int nst = 0;
+  unsigned read = 0, written = 0; // of the warp
   for (;;) {
     // new records once fetch_min lanes are idle (or all are: the last ones)
     const unsigned need = __ballot_sync(0xffffffffu, !have);
@@ -269,12 +254,10 @@ template <class R, int PT, int K> __device__ __forceinline__ void transport_body
           gxs.have = 0; // a new photon energy
         }
       }
-      // records read: counted per warp (no per-thread counters held across
-      // the loop; the host adds them to the type's total of records read)
-      if ((int)lane_id() == leader) {
-        const long long got = min((long long)__popc(need), n - (long long)base);
-        if (got > 0) atomicAdd(&sm_stat[S_TREAD0 + PT], (unsigned long long)got);
-      }
+      // records read and written: counted per warp, in registers (the host adds
+      // them to the type's totals; those queued for interactions are counted by
+      // k_finish from the buffers' counters)
+      read += (unsigned)max(0LL, min((long long)__popc(need), n - (long long)base));
       if ((long long)base + __popc(need) >= n) more = false;
     }
     if (!__any_sync(0xffffffffu, have)) break;
@@ -295,13 +278,24 @@ template <class R, int PT, int K> __device__ __forceinline__ void transport_body
     }
     const bool w_alive = done && r == kAlive && nst >= budget;
     const bool w_int = done && r == kInteract;
-    const long long slot = warp_take1((unsigned long long *)&ctl->count[par ^ 1][PT], w_alive);
-    long long q = 0;
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-      if (PT == 1 && p == 2) continue; // e- has two processes
-      const long long v = warp_take1((unsigned long long *)&ctl->qcount[PT][p], w_int && proc == p);
-      if (p == proc) q = v;
+    // slots in the next store and the interaction buffers, one per lane that
+    // needs one: lane k adds to counter k (store, processes 0 to 2), the
+    // additions in flight together
+    const unsigned m_al = __ballot_sync(0xffffffffu, w_alive), m0 = __ballot_sync(0xffffffffu, w_int && proc == 0),
+                   m1 = __ballot_sync(0xffffffffu, w_int && proc == 1),
+                   m2 = PT == 1 ? 0u : __ballot_sync(0xffffffffu, w_int && proc == 2);
+    const unsigned wr = m_al | m0 | m1 | m2;
+    long long slot = 0, q = 0;
+    if (wr) {
+      const int k = (int)lane_id();
+      const int mine = k > 3 ? 0 : __popc(k == 0 ? m_al : (k == 1 ? m0 : (k == 2 ? m1 : m2)));
+      unsigned long long base = 0;
+      if (mine)
+        base = atomicAdd((unsigned long long *)(k == 0 ? &ctl->count[par ^ 1][PT] : &ctl->qcount[PT][k - 1]),
+                         (unsigned long long)mine);
+      base = __shfl_sync(0xffffffffu, base, w_int ? proc + 1 : 0);
+      const unsigned with = w_int ? (proc == 0 ? m0 : (proc == 1 ? m1 : m2)) : m_al;
+      slot = q = (long long)base + __popc(with & lanemask_lt());
     }
     bool queued = false;
     if (w_alive) {
@@ -316,12 +310,12 @@ template <class R, int PT, int K> __device__ __forceinline__ void transport_body
         L.deposit(t.event, t.vol, (double)t.E);
       }
     }
-    // records written (to the next store or an interaction buffer), per warp;
-    // those queued for interactions are counted by k_finish from the buffers'
-    // counters, and the host adds these to the type's total of records written
-    const unsigned wr = __ballot_sync(0xffffffffu, w_alive || queued);
-    if (lane_id() == 0 && wr) atomicAdd(&sm_stat[S_TWRITE0 + PT], (unsigned long long)__popc(wr));
+    written += __popc(__ballot_sync(0xffffffffu, w_alive || queued));
     if (done && (r != kAlive || nst >= budget)) have = false;
+  }
+  if (lane_id() == 0) {
+    if (read) atomicAdd(&sm_stat[S_TREAD0 + PT], (unsigned long long)read);
+    if (written) atomicAdd(&sm_stat[S_TWRITE0 + PT], (unsigned long long)written);
   }
   tally_end(L, ctl, a.edep, sm_edep, sm_stat, sm_esc, &sm_err, S_TSTEP0 + PT);
   GX_TL_END();
@@ -1029,7 +1023,7 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
   L.block = cfg->block_size > 0 ? cfg->block_size : default_block(cfg->engine);
   int bpsm = cfg->blocks_per_sm > 0 ? cfg->blocks_per_sm : default_blocks_per_sm(*cfg);
   L.grid = C->num_sms * bpsm;
-  L.smem = 768 * sizeof(double);
+  L.smem = kTallyDoubles * sizeof(double);
 
   if (nprim > E->cumE_cap) {
     if (E->cumE) cudaFree(E->cumE);
@@ -1867,7 +1861,7 @@ extern "C" int gx_transport_run_noalloc(gx_ctx *ctx, const gx_transport_config *
   L.a.refill_below = cfg->refill_below > 0 ? std::min(cfg->refill_below, cap) : cap / 2;
   L.block = cfg->block_size > 0 ? cfg->block_size : 256;
   L.grid = C->num_sms * (cfg->blocks_per_sm > 0 ? cfg->blocks_per_sm : 4);
-  L.smem = 768 * sizeof(double);
+  L.smem = kTallyDoubles * sizeof(double);
 
   // the control block starts from zero on every call
   Ctl h;
