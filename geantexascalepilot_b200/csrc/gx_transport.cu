@@ -646,6 +646,9 @@ struct Engine {
   void *dargs = nullptr; // device copy of the launch arguments (batched engine)
   cudaStream_t s1 = nullptr, s2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_j1 = nullptr, ev_j2 = nullptr;
+  // per particle type: branches for its second and third interaction kernel
+  cudaStream_t side[3][2] = {};
+  cudaEvent_t side_fork[3] = {}, side_join[3][2] = {};
 };
 
 void release_engine(Ctx *c)
@@ -664,6 +667,13 @@ void release_engine(Ctx *c)
   if (e->ev_fork) cudaEventDestroy(e->ev_fork);
   if (e->ev_j1) cudaEventDestroy(e->ev_j1);
   if (e->ev_j2) cudaEventDestroy(e->ev_j2);
+  for (int q = 0; q < 3; ++q) {
+    if (e->side_fork[q]) cudaEventDestroy(e->side_fork[q]);
+    for (int k = 0; k < 2; ++k) {
+      if (e->side[q][k]) cudaStreamDestroy(e->side[q][k]);
+      if (e->side_join[q][k]) cudaEventDestroy(e->side_join[q][k]);
+    }
+  }
   delete e;
   GX_ENGINE_OF(c) = nullptr;
 }
@@ -756,12 +766,31 @@ template <class R, int PT, int PROC> static void (*interact_for(const Launch<R> 
   return k_interact<R, PT, PROC>;
 }
 
-// One type's interaction kernels (gamma 3 processes, e- 2, e+ 3).
-template <class R, int PT> static void enqueue_interactions(const Launch<R> &L, const Args<R> *A, cudaStream_t s)
+// One type's interaction kernels (gamma 3 processes, e- 2, e+ 3): one after
+// another, or (e given) the second and third on branches of their own beside
+// the first.  They read different buffers and reserve their outputs by atomics;
+// with few tracks each is 20 us of latency whatever its work: 61 showers 13.9 ms
+// in a row, 12.5 side by side, two electrons 4.8 and 4.0, a full batch of 20000
+// 136.0 and 135.2.
+template <class R, int PT>
+static void enqueue_interactions(const Launch<R> &L, const Args<R> *A, cudaStream_t s, Engine *e = nullptr)
 {
-  interact_for<R, PT, 0>(L)<<<L.grid, L.block, L.smem, s>>>(A);
-  interact_for<R, PT, 1>(L)<<<L.grid, L.block, L.smem, s>>>(A);
-  if constexpr (PT != 1) interact_for<R, PT, 2>(L)<<<L.grid, L.block, L.smem, s>>>(A);
+  cudaStream_t to[3] = {s, s, s};
+  if (e) {
+    cudaEventRecord(e->side_fork[PT], s);
+    for (int k = 0; k < (PT == 1 ? 1 : 2); ++k) {
+      to[k + 1] = e->side[PT][k];
+      cudaStreamWaitEvent(to[k + 1], e->side_fork[PT], 0);
+    }
+  }
+  interact_for<R, PT, 0>(L)<<<L.grid, L.block, L.smem, to[0]>>>(A);
+  interact_for<R, PT, 1>(L)<<<L.grid, L.block, L.smem, to[1]>>>(A);
+  if constexpr (PT != 1) interact_for<R, PT, 2>(L)<<<L.grid, L.block, L.smem, to[2]>>>(A);
+  if (e)
+    for (int k = 0; k < (PT == 1 ? 1 : 2); ++k) {
+      cudaEventRecord(e->side_join[PT][k], to[k + 1]);
+      cudaStreamWaitEvent(s, e->side_join[PT][k], 0);
+    }
 }
 
 // One iteration.  interact: this iteration runs the interaction kernels (the
@@ -795,11 +824,11 @@ static void enqueue_iteration(const Launch<R> &L, Engine *e, cudaStream_t s, boo
   // about one record per lane, then three interaction kernels) is the one
   // that ends an iteration most often when it is dispatched last.
   transport_for<R, 2>(L)<<<L.grid, L.block, L.smem, sp>>>(A);
-  if (interact) enqueue_interactions<R, 2>(L, A, sp);
+  if (interact) enqueue_interactions<R, 2>(L, A, sp, concurrent ? e : nullptr);
   transport_for<R, 1>(L)<<<L.grid, L.block, L.smem, se>>>(A);
-  if (interact) enqueue_interactions<R, 1>(L, A, se);
+  if (interact) enqueue_interactions<R, 1>(L, A, se, concurrent ? e : nullptr);
   transport_for<R, 0>(L)<<<L.grid, L.block, L.smem, sg>>>(A);
-  if (interact) enqueue_interactions<R, 0>(L, A, sg);
+  if (interact) enqueue_interactions<R, 0>(L, A, sg, concurrent ? e : nullptr);
   if (concurrent) {
     cudaEventRecord(e->ev_j1, e->s1);
     cudaEventRecord(e->ev_j2, e->s2);
@@ -944,6 +973,13 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
     cudaEventCreateWithFlags(&E->ev_fork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&E->ev_j1, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&E->ev_j2, cudaEventDisableTiming);
+    for (int q = 0; q < 3; ++q) {
+      cudaEventCreateWithFlags(&E->side_fork[q], cudaEventDisableTiming);
+      for (int k = 0; k < 2; ++k) {
+        cudaStreamCreateWithFlags(&E->side[q][k], cudaStreamNonBlocking);
+        cudaEventCreateWithFlags(&E->side_join[q][k], cudaEventDisableTiming);
+      }
+    }
   }
   Launch<R> L;
   std::memset(&L.a, 0, sizeof(L.a));
