@@ -257,6 +257,8 @@ static void append_coeffs(const HostVec &v, std::vector<double> &C64, std::vecto
       C64.push_back(c[k]);
       C32.push_back((float)c[k]);
     }
+    C32.push_back(0.0f); // to 32 bytes
+    C32.push_back(0.0f);
   }
 }
 
@@ -281,7 +283,7 @@ int refit_vector(Ctx *ctx, int table, int mat, const double *ynew)
       (e = cudaMemcpy(const_cast<double *>(d.d2) + vd.off, v.d2.data(), n * sizeof(double), cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(const_cast<double *>(d.c64) + 6 * vd.off, C64.data(), C64.size() * sizeof(double),
                       cudaMemcpyHostToDevice)) ||
-      (e = cudaMemcpy(const_cast<float *>(d.c32) + 6 * vd.off, C32.data(), C32.size() * sizeof(float),
+      (e = cudaMemcpy(const_cast<float *>(d.c32) + 8 * vd.off, C32.data(), C32.size() * sizeof(float),
                       cudaMemcpyHostToDevice)))
     return cuda_error(e, "refit: upload");
   return GX_OK;
