@@ -84,8 +84,16 @@ inline int default_blocks_per_sm(const gx_transport_config &c)
   return c.engine == 1 && c.precision == 1 && plain ? 5 : kDefaultBlocksPerSM;
 }
 // Steps of one track per transport-kernel launch in the batched engine, at
-// most (a track is kept in registers while it neither interacts nor dies).
-constexpr int kDefaultStepsPerLaunch = 16;
+// most (a track is kept in registers while it neither interacts nor dies), for
+// gamma, e-, e+.  A launch ends with its slowest track, and a pass of a warp is
+// about 3 us of latency: long turns pay where the launch has many tracks for
+// each lane (a written record less), short ones where it has not, since every
+// track waits for the one that takes the most steps.  Measured (ms) with 16 steps
+// (e+ 4) throughout, with kDefaultSteps, and with kFewSteps below one track per
+// thread: 61 showers 12.6, 11.3, 9.3; two electrons 3.98, 3.97, 3.65; 10^4
+// electrons in FP64 17.5, 16.9, 16.3; 20000 showers 131.5, 130.8, 129.6.  Fewer
+// steps of e- or e+ (1) or of photons (4) lost everywhere.
+constexpr int kDefaultSteps[3] = {16, 4, 2}, kFewSteps[3] = {6, 2, 2};
 // Idle lanes of a warp before it takes new records in the transport kernel of
 // type q (0 gamma, 1 e-, 2 e+).  Measured: the FP32-mixed photon kernels of the
 // layered geometry gain 1.9% on C3, 2.7% on C4 and 0.9% with multiple

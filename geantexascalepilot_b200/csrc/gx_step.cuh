@@ -111,7 +111,9 @@ template <class R> struct Args {
   // compactly so the interaction kernels read them coalesced (batched engine)
   Store<R> ibuf[3][3];
   long long qcap;
-  int step_budget[3]; // steps of one track per transport launch, at most, per particle type
+  // steps of one track per transport launch, at most, per particle type; few: when
+  // the store has no more tracks than the grid has threads
+  int step_budget[3], few_budget[3];
   int fetch_min[3];   // idle lanes of a warp before it takes new records, per particle type
 };
 

@@ -287,7 +287,8 @@ typedef struct {
   double wave_energy;      /* energy (MeV) carried by live tracks before more primaries are injected,
                               at most (0: from capacity) */
   int steps_per_launch;    /* batched engine: steps of one track per transport launch, at most; a track
-                              stays in registers between them (0: default 16; 1: one step per iteration) */
+                              stays in registers between them (0: the engine's own choice, by particle type
+                              and by how many tracks there are; 1: one step per iteration) */
   int msc;                 /* 1: multiple scattering of e-/e+ (Urban-type: safety-based step limit, true /
                               geometric path conversion, angular deflection); 2: the same with lateral
                               displacement (within the safety); 0: off (the reference has none,
@@ -295,7 +296,8 @@ typedef struct {
   int field_map;           /* 1: the context's field map (gx_ctx_load_field_map) with fourth-order
                               Runge-Kutta sub-steps, Bz ignored; 0: uniform Bz with the helix */
   int steps_per_launch_by_type[3]; /* batched engine: steps per transport launch for gamma, e-, e+
-                              (0: from steps_per_launch; e+ a quarter of it, at least 1) */
+                              (0: from steps_per_launch, e+ a quarter of it, at least 1; both 0: the
+                              engine's own choice) */
   int interaction_interval; /* batched engine: the compaction interval -- tracks that reach an interaction wait
                               in their per-process buffers and the interaction kernels, which compact their
                               survivors and secondaries back into the stores, run every this many iterations
