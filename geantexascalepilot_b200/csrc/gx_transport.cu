@@ -421,13 +421,15 @@ __global__ void __launch_bounds__(1024, 1) k_interact_wide(const Args<R> *__rest
   interact_body<R, PT, PROC>(A);
 }
 
-// End of an iteration: the next stores become current, the refill plan for
-// the following iteration is made.  One thread.  interacted: the interaction
-// kernels ran in this iteration (their buffers are emptied); otherwise the
-// tracks waiting in them count as pending.
-__global__ void k_finish(Ctl *ctl, long long cap0, long long cap1, long long cap2, int nstores, int interacted)
+// End of an iteration: the refill that opened it is booked, the next stores
+// become current, the refill plan for the following iteration is made.
+// interacted: the interaction kernels ran in this iteration (their buffers are
+// emptied); otherwise the tracks waiting in them count as pending.
+__device__ void finish_iteration(Ctl *ctl, long long cap0, long long cap1, long long cap2, int nstores, int interacted)
 {
-  GX_TL_BEGIN(ctl, 14);
+  for (int q = 0; q < 3; ++q) ctl->take_stack[q] = 0;
+  ctl->prim_next += ctl->take_prim;
+  ctl->take_prim = 0;
   int par = ctl->parity, np = par ^ 1;
   const long long cap[3] = {cap0, cap1, cap2};
   const long long refill_below = ctl->refill_below, stack_cap = ctl->stack_cap;
@@ -498,6 +500,25 @@ __global__ void k_finish(Ctl *ctl, long long cap0, long long cap1, long long cap
   ctl->in_flight = fl;
   ctl->pending = pend;
   if (fl > ctl->peak) ctl->peak = fl;
+}
+
+// One thread's work, on a copy of the control block in shared memory that the
+// block reads and writes together: word by word from L2 it took 4.2 us of every
+// iteration, and the booking of the refill was a launch of its own.
+constexpr int kFinishBlock = 128;
+__global__ void __launch_bounds__(kFinishBlock) k_finish(Ctl *ctl, long long cap0, long long cap1, long long cap2,
+                                                         int nstores, int interacted)
+{
+  __shared__ Ctl c;
+  static_assert(sizeof(Ctl) % 8 == 0, "copied as 64-bit words");
+  GX_TL_BEGIN(ctl, 14);
+  for (int k = threadIdx.x; k < (int)(sizeof(Ctl) / 8); k += kFinishBlock)
+    reinterpret_cast<unsigned long long *>(&c)[k] = reinterpret_cast<const unsigned long long *>(ctl)[k];
+  __syncthreads();
+  if (threadIdx.x == 0) finish_iteration(&c, cap0, cap1, cap2, nstores, interacted);
+  __syncthreads();
+  for (int k = threadIdx.x; k < (int)(sizeof(Ctl) / 8); k += kFinishBlock)
+    reinterpret_cast<unsigned long long *>(ctl)[k] = reinterpret_cast<const unsigned long long *>(&c)[k];
   GX_TL_END();
 }
 
@@ -525,15 +546,19 @@ __global__ void __launch_bounds__(1024) k_prefix_energy(const double *__restrict
   }
 }
 
-__device__ __forceinline__ void jump_matvec(const uint64_t *A, uint64_t v[3], uint64_t m)
+// v := A v modulo m = 2^32 - c (the folding of k_rng_substreams' products)
+__device__ __forceinline__ void jump_matvec(const uint64_t *A, uint64_t v[3], uint32_t c, uint32_t m)
 {
   uint64_t r[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     uint64_t acc = 0;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) acc = ((A[3 * i + k] * v[k]) % m + acc) % m;
-    r[i] = acc;
+    for (int k = 0; k < 3; ++k) {
+      const uint64_t x = A[3 * i + k] * v[k];
+      acc += (x >> 32) * c + (x & 0xffffffffull);
+    }
+    r[i] = Mrg::mod_m(acc, c, m);
   }
   v[0] = r[0];
   v[1] = r[1];
@@ -607,8 +632,8 @@ template <class R> __device__ __forceinline__ void refill_body(const Args<R> &a)
       uint64_t v2[3] = {(uint64_t)a.p.seed[3], (uint64_t)a.p.seed[4], (uint64_t)a.p.seed[5]};
       for (int b = 0; kk != 0 && b < 64; ++b, kk >>= 1)
         if (kk & 1ULL) {
-          jump_matvec(a.p.jump + 9 * b, v1, 4294967087ULL);
-          jump_matvec(a.p.jump + 9 * (64 + b), v2, 4294944443ULL);
+          jump_matvec(a.p.jump + 9 * b, v1, Mrg::kC1, Mrg::kM1u);
+          jump_matvec(a.p.jump + 9 * (64 + b), v2, Mrg::kC2, Mrg::kM2u);
         }
       for (int k = 0; k < 3; ++k) {
         t.rs[k] = (uint32_t)v1[k];
@@ -641,7 +666,8 @@ template <class R> __global__ void __launch_bounds__(1024) k_refill_p(const Args
   GX_TL_END();
 }
 
-// Bookkeeping after a refill: the primary cursor.  One thread.
+// Bookkeeping after a refill that no iteration follows (the hand-over of live
+// tracks): the primary cursor.  One thread.
 __global__ void k_refill_done(Ctl *ctl)
 {
   GX_TL_BEGIN(ctl, 1);
@@ -831,13 +857,11 @@ static void enqueue_iteration(const Launch<R> &L, Engine *e, cudaStream_t s, boo
   if (L.a.nstores == 1) {
     // plain loop: one fused step kernel over the mixed store
     k_refill_p<R><<<L.grid, L.block, 0, s>>>(A);
-    k_refill_done<<<1, 1, 0, s>>>(L.a.ctl);
     step_kernel_p<R>(kernel_kind<R>(L.a.g))<<<L.grid, L.block, L.smem, s>>>(A);
-    k_finish<<<1, 1, 0, s>>>(L.a.ctl, L.a.st[0][0].cap, L.a.st[0][1].cap, L.a.st[0][2].cap, L.a.nstores, 1);
+    k_finish<<<1, kFinishBlock, 0, s>>>(L.a.ctl, L.a.st[0][0].cap, L.a.st[0][1].cap, L.a.st[0][2].cap, L.a.nstores, 1);
     return;
   }
   k_refill_p<R><<<L.grid, L.block, 0, s>>>(A);
-  k_refill_done<<<1, 1, 0, s>>>(L.a.ctl);
   cudaStream_t sg = s, se = s, sp = s;
   if (concurrent) {
     // gamma on s, e- on s1, e+ on s2
@@ -864,7 +888,7 @@ static void enqueue_iteration(const Launch<R> &L, Engine *e, cudaStream_t s, boo
     cudaStreamWaitEvent(s, e->ev_j1, 0);
     cudaStreamWaitEvent(s, e->ev_j2, 0);
   }
-  k_finish<<<1, 1, 0, s>>>(L.a.ctl, L.a.st[0][0].cap, L.a.st[0][1].cap, L.a.st[0][2].cap, L.a.nstores,
+  k_finish<<<1, kFinishBlock, 0, s>>>(L.a.ctl, L.a.st[0][0].cap, L.a.st[0][1].cap, L.a.st[0][2].cap, L.a.nstores,
                            interact ? 1 : 0);
 }
 
@@ -1114,7 +1138,7 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
   err = cudaMemcpyAsync(E->ctl, &h, sizeof(Ctl), cudaMemcpyHostToDevice, s);
   if (err != cudaSuccess) return cuda_error(err, "transport control init");
   // first refill plan
-  k_finish<<<1, 1, 0, s>>>(E->ctl, cap, cap, cap, nstores, 1);
+  k_finish<<<1, kFinishBlock, 0, s>>>(E->ctl, cap, cap, cap, nstores, 1);
   cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
   cudaEventCreate(&t1);
@@ -1145,7 +1169,6 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
     for (;;) {
       if (cfg->profile) {
         k_refill_p<R><<<L.grid, L.block, 0, s>>>((const Args<R> *)E->dargs);
-        k_refill_done<<<1, 1, 0, s>>>(L.a.ctl);
         for (int q = 0; q < nstores; ++q) {
           cudaEventRecord(ea[q], s);
           if (!batched) {
@@ -1157,7 +1180,7 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
           }
           cudaEventRecord(eb[q], s);
         }
-        k_finish<<<1, 1, 0, s>>>(L.a.ctl, L.a.st[0][0].cap, L.a.st[0][1].cap, L.a.st[0][2].cap, L.a.nstores,
+        k_finish<<<1, kFinishBlock, 0, s>>>(L.a.ctl, L.a.st[0][0].cap, L.a.st[0][1].cap, L.a.st[0][2].cap, L.a.nstores,
                                  (iters + 1) % every == 0 ? 1 : 0);
       } else {
         enqueue_iteration(L, E, s, false, (iters + 1) % every == 0);
@@ -1945,15 +1968,14 @@ extern "C" int gx_transport_run_noalloc(gx_ctx *ctx, const gx_transport_config *
       (err = cudaStreamSynchronize(s)) != cudaSuccess)
     return cuda_error(err, "gx_transport_run_noalloc: control block");
   if (nprim > 0) k_prefix_energy<<<1, 1024, 0, s>>>(d_E, nprim, cumE, nullptr);
-  k_finish<<<1, 1, 0, s>>>(ctl, cap, cap, cap, 1, 1);
+  k_finish<<<1, kFinishBlock, 0, s>>>(ctl, cap, cap, cap, 1, 1);
   Ctl hc;
   long long iters = 0;
   for (;;) {
     k_refill<double><<<L.grid, L.block, 0, s>>>(L.a);
-    k_refill_done<<<1, 1, 0, s>>>(ctl);
     (cfg->msc ? (cfg->field_map ? k_step<double, 3, 5> : k_step<double, 3, 4>)
               : (cfg->field_map ? k_step<double, 3, 1> : k_step<double, 3, 0>))<<<L.grid, L.block, L.smem, s>>>(L.a);
-    k_finish<<<1, 1, 0, s>>>(ctl, cap, cap, cap, 1, 1);
+    k_finish<<<1, kFinishBlock, 0, s>>>(ctl, cap, cap, cap, 1, 1);
     if ((err = cudaGetLastError()) != cudaSuccess) return cuda_error(err, "gx_transport_run_noalloc: launch");
     if ((err = cudaMemcpyAsync(&hc, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (err = cudaStreamSynchronize(s)) != cudaSuccess)
