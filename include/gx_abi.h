@@ -282,7 +282,8 @@ typedef struct {
                               batched engine, 4 otherwise) */
   long long capacity;      /* track slots per particle type (0: default) */
   long long refill_below;  /* inject / refill when fewer tracks than this are in flight (0: default) */
-  int graph_iters;         /* iterations per CUDA-graph launch between host checks (0: default) */
+  int graph_iters;         /* iterations per CUDA-graph launch between host checks (0: the graph repeats
+                              by itself while tracks are left) */
   int profile;             /* 1: no graph; CUDA events around every step kernel (per-kernel times in stats) */
   double wave_energy;      /* energy (MeV) carried by live tracks before more primaries are injected,
                               at most (0: from capacity) */
