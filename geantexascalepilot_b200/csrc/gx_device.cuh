@@ -642,7 +642,12 @@ __device__ int sg_sample(Mrg &r, const Data &d, const ModelParams &p, Inter<R> &
     int it = 0;
     do {
       R q = r.u<R>();
-      z = R(2) * A * (R(2) * q + Ap2 * M<R>::sqrt(q)) / (Ap2 * Ap2 - R(4) * q);
+      // which product of the sums is fused is fixed here: left open, it differed
+      // from kernel to kernel, and a float's last bit is another track
+      if constexpr (sizeof(R) == 4)
+        z = R(2) * A * __fmaf_rn(Ap2, sqrtf(q), 2.0f * q) / __fmaf_rn(Ap2, Ap2, -4.0f * q);
+      else
+        z = R(2) * A * (R(2) * q + Ap2 * M<R>::sqrt(q)) / (Ap2 * Ap2 - R(4) * q);
       g = (R(2) - z) * (R(1) / (A + z) + B);
       if (++it > kRejectCap) {
         *err |= kErrRejectCap;

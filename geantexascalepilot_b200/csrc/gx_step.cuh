@@ -818,6 +818,27 @@ __device__ __noinline__ double3 msc_displacement(const Geom &g, int vol, double 
   return out;
 }
 
+#ifndef GX_PARITY
+// Whether an electron of energy e that starts at pos in volume vol comes to rest
+// in its first step there unless it interacts: its step limit is its range (the
+// range is below the step function's final range) and nothing of the volume's
+// surface is within it.  Such a step is one straight or helix move that stays in
+// the volume and deposits all of e there, whatever the direction (step_gpil,
+// field_substep: safety above the remaining length; along_loss: step >= range).
+// The margin is far above the move's rounding and the navigator's snap distance.
+// range: the step.
+template <class R>
+__device__ __forceinline__ bool stops_at_once(const Data &d, const Geom &g, int vol, const double *pos, int mat, R e,
+                                              R &range)
+{
+  R raw;
+  range = range_limit<R>(d, 1, mat, e, raw);
+  const R cut = (R)d.cut_length[1][mat], finR = (R(10.0) < cut) ? R(10.0) : cut;
+  if (e < R(kMinE)) raw *= e / R(kMinE);
+  return raw <= finR && safety(g, vol, pos) > 1.0001 * (double)range + 2e-6;
+}
+#endif
+
 enum { kDone = 0, kAlive = 1, kInteract = 2 };
 
 // One OneStep (test_BasicCpuTransport.cpp:408-497 / InnerStep :358-403) in

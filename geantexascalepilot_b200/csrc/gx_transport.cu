@@ -368,6 +368,98 @@ template <class R, int PT, int K> __global__ void __launch_bounds__(1024, 1) k_t
   transport_body<R, PT, K>(A);
 }
 
+#ifndef GX_PARITY
+// Electrons that stops_at_once() finds to end in the volume they are created in never become
+// records: about half of all e- steps are the only step of a photo-electron or a
+// Compton electron, and it leaves nothing but its deposit and its counts.  In
+// the layered or box geometry, without multiple scattering, and with enough of
+// them (n, the interactions of a launch) that throughput counts: 20000 showers
+// 128.9 to 123.7 ms, 256 events 169.8 to 163.7, but two electrons 3.06 to 3.16,
+// where the looking is latency on the way to the next iteration.
+__device__ __forceinline__ bool local_stops(const Geom &g, long long n)
+{
+  return !g.msc && g.geometry != 2 && !g.charged_local && n >= 1024;
+}
+
+template <class R> __device__ __forceinline__ void book_stop(const Geom &g, const Track<R> &t, R e, Local &L)
+{
+  L.deposit(t.event, t.vol, (double)e);
+  L.st[S_SEC1]++;
+  L.st[S_STEPS]++;
+  if (g.Bz != 0.0 || g.field_map) L.st[S_SUBSTEPS]++;
+}
+
+// The photo-electron of photon t, when it stops at once and no process can come
+// before (no cross section at its energy): its energy and the shell's are
+// deposited, and neither its direction nor its stream is sampled, since nothing
+// is left that would use them.
+template <class R> __device__ __forceinline__ bool photo_electron_stops(const Data &d, const Geom &g, Track<R> &t, Local &L)
+{
+  const int mat = vol_material(g, t.vol);
+  const R e = (R)photo_electron_energy(d, (int)d.mat_Z[mat], (double)t.E, 1);
+  if (!(e > R(0)) || (double)e > d.vec[GX_Lambda_eIoni_em][mat].emin || (double)e > d.vec[GX_Lambda_eBrem_em][mat].emin)
+    return false;
+  R range;
+  if (!stops_at_once<R>(d, g, t.vol, t.pos, mat, e, range)) return false;
+  L.deposit(t.event, t.vol, (double)(t.E - e));
+  book_stop(g, t, e, L);
+  t.E = R(0);
+  return true;
+}
+
+// emit_tracks for a Compton scattering or photo-electric absorption (at most one
+// electron, in the batched engine's three stores): the electron is booked on the
+// spot when `local` and it stops at once before any interaction.
+template <class R>
+__device__ __forceinline__ void emit_electron(const Args<R> &a, Ctl *ctl, int par, bool active, bool alive, Track<R> &t,
+                                              const Secs<R> &sec, bool local, Local &L)
+{
+  const bool child = active && sec.n == 1;
+  bool stop = false;
+  Track<R> c = t;
+  if (active) {
+    Mrg rng = t.rng();
+    if (child) {
+      c.type = 1;
+      c.dir[0] = sec.dir[0][0];
+      c.dir[1] = sec.dir[0][1];
+      c.dir[2] = sec.dir[0][2];
+      c.E = sec.E[0];
+      c.nil[0] = c.nil[1] = c.nil[2] = R(-1);
+      c.msc_r0 = R(-1);
+      c.prim = -1;
+      Mrg cr;
+      rng.seed_child(cr);
+      draw_nils(c, cr);
+      c.set_rng(cr);
+      const int mat = vol_material(a.g, c.vol);
+      R range;
+      if (local && stops_at_once<R>(*a.d, a.g, c.vol, c.pos, mat, c.E, range)) {
+        // as step_gpil chooses: a process comes first unless its length is above the range
+        R xs[3];
+        cross_sections<R>(*a.d, 1, mat, c.E, xs);
+        stop = true;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (xs[i] > R(0) && !(range < c.nil[i] / xs[i])) stop = false;
+      }
+      if (stop)
+        book_stop(a.g, t, c.E, L);
+      else
+        L.st[S_SEC1]++;
+    }
+    if (alive) draw_nils(t, rng);
+    t.set_rng(rng);
+  }
+  const int cnt[3] = {alive ? 1 : 0, child && !stop ? 1 : 0, 0};
+  long long next[3];
+  warp_reserve3((unsigned long long *)ctl->count[par ^ 1], 2, cnt, next);
+  if (cnt[1]) put_track(a, 1, next[1], c, L);
+  if (cnt[0]) put_track(a, 0, next[0], t, L);
+  L.st[S_WRITE0] += cnt[0] + cnt[1];
+}
+#endif
+
 // Post-step interaction of process PROC for the buffered tracks of type PT:
 // one model per kernel, so a warp runs one sampling algorithm; survivor and
 // secondaries go to the next stores.
@@ -390,6 +482,9 @@ template <class R, int PT, int PROC> __device__ __forceinline__ void interact_bo
   }
   Local L;
   tally_begin(L, a.g, a.edep, sm_edep, sm_stat, sm_esc, &sm_err);
+#ifndef GX_PARITY
+  const bool local = local_stops(a.g, n);
+#endif
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long base = (long long)blockIdx.x * blockDim.x; base < n; base += stride) {
     long long j = base + threadIdx.x;
@@ -401,12 +496,23 @@ template <class R, int PT, int PROC> __device__ __forceinline__ void interact_bo
     if (active) {
       load_track(buf, j, PT, t);
       L.st[S_READ0 + PT]++;
-      run_model(d, a.g, t, PROC, sec, L);
-      alive = t.E > R(0);
+      bool sample = true;
+#ifndef GX_PARITY
+      if (PT == 0 && PROC == 2 && local) sample = !photo_electron_stops(d, a.g, t, L);
+#endif
+      if (sample) {
+        run_model(d, a.g, t, PROC, sec, L);
+        alive = t.E > R(0);
+      }
     }
-    emit_tracks<R, PT>(a, ctl, par, active, alive, t, sec, L);
+#ifndef GX_PARITY
+    if constexpr (PT == 0 && PROC != 1)
+      emit_electron(a, ctl, par, active, alive, t, sec, local, L);
+    else
+#endif
+      emit_tracks<R, PT>(a, ctl, par, active, alive, t, sec, L);
   }
-  tally_end(L, ctl, a.edep, sm_edep, sm_stat, sm_esc, &sm_err);
+  tally_end(L, ctl, a.edep, sm_edep, sm_stat, sm_esc, &sm_err, S_TSTEP1);
   GX_TL_END();
 }
 
