@@ -197,6 +197,8 @@ __device__ __forceinline__ void timeline_mark(int slot, int end)
 #define GX_TL_END()
 #endif
 
+constexpr int kPhotonSteps = 4;
+
 // Transport of the tracks of type PT: each lane keeps its track in registers
 // and steps it until the track interacts (it then goes to the interaction
 // buffer of its process), dies, leaves the world, or has taken step_budget
@@ -292,18 +294,35 @@ template <class R, int PT, int K> __device__ __forceinline__ void transport_body
     if (!__any_sync(0xffffffffu, have)) break;
     int r = kDone, proc = -1;
     bool done = false; // a step ends in this pass
-    if (have && !infield) {
-      infield = step_begin<R, K>(d, a.g, t, c, PT == 0 ? &gxs : nullptr);
-      done = !infield;
-    }
-    if (PT != 0 && have && infield && field_substep<R, K>(d, a.g, t, c, L)) {
-      infield = false;
-      done = true;
-    }
-    if (done) {
-      r = step_end<R, K>(d, a.g, t, c, L, &proc);
-      ++nst;
-      if (t.prim >= 0 && a.pstep) atomicAdd(&a.pstep[t.prim], 1);
+    if constexpr (PT == 0) {
+      // A photon's step is short (most cross a slab with the cross sections it
+      // has), so a pass takes up to kPhotonSteps of them before the warp looks for
+      // new records and results again: 20000 showers 123.9 ms with 1, 123.2 with
+      // 2, 122.3 with 4; at 8 the lanes that are done wait too long (128.0).
+      if (have) {
+#pragma unroll 1
+        for (int k = 0; k < kPhotonSteps && !(done && (r != kAlive || nst >= budget)); ++k) {
+          step_begin<R, K>(d, a.g, t, c, &gxs);
+          r = step_end<R, K>(d, a.g, t, c, L, &proc);
+          done = true;
+          ++nst;
+          if (t.prim >= 0 && a.pstep) atomicAdd(&a.pstep[t.prim], 1);
+        }
+      }
+    } else {
+      if (have && !infield) {
+        infield = step_begin<R, K>(d, a.g, t, c);
+        done = !infield;
+      }
+      if (have && infield && field_substep<R, K>(d, a.g, t, c, L)) {
+        infield = false;
+        done = true;
+      }
+      if (done) {
+        r = step_end<R, K>(d, a.g, t, c, L, &proc);
+        ++nst;
+        if (t.prim >= 0 && a.pstep) atomicAdd(&a.pstep[t.prim], 1);
+      }
     }
     const bool w_alive = done && r == kAlive && nst >= budget;
     const bool w_int = done && r == kInteract;
