@@ -566,11 +566,21 @@ __device__ __forceinline__ void helix_bz(T rn, T sB, double s, const double pos[
   T sh, ch;
   sincos_t(T(0.5) * phi, &sh, &ch);
   const T sinp = T(2) * sh * ch, cm1 = T(-2) * sh * sh, cosp = T(1) + cm1;
-  np[0] = pos[0] + (double)(rn * (cm1 * dir[1] * sB - sinp * dir[0]));
-  np[1] = pos[1] + (double)(rn * (-cm1 * dir[0] * sB - sinp * dir[1]));
   np[2] = pos[2] + s * (double)dir[2];
-  nd[0] = cosp * dir[0] + sinp * dir[1] * sB;
-  nd[1] = cosp * dir[1] - sinp * dir[0] * sB;
+  // FP32: which product of a sum is fused is written out; left open it differed
+  // from kernel to kernel, and a float's last bit is another track
+  if constexpr (sizeof(T) == 4) {
+    const float P = __fmul_rn(sinp, dir[0]), Q = __fmul_rn(sinp, dir[1]);
+    np[0] = pos[0] + (double)(rn * __fmaf_rn(__fmul_rn(cm1, dir[1]), sB, -P));
+    np[1] = pos[1] + (double)(rn * __fmaf_rn(__fmul_rn(-cm1, dir[0]), sB, -Q));
+    nd[0] = __fmaf_rn(cosp, dir[0], __fmul_rn(Q, sB));
+    nd[1] = __fmaf_rn(cosp, dir[1], -__fmul_rn(P, sB));
+  } else {
+    np[0] = pos[0] + (double)(rn * (cm1 * dir[1] * sB - sinp * dir[0]));
+    np[1] = pos[1] + (double)(rn * (-cm1 * dir[0] * sB - sinp * dir[1]));
+    nd[0] = cosp * dir[0] + sinp * dir[1] * sB;
+    nd[1] = cosp * dir[1] - sinp * dir[0] * sB;
+  }
   nd[2] = dir[2];
 }
 
@@ -1165,7 +1175,12 @@ __device__ __forceinline__ bool field_substep(const Data &d, const Geom &g, Trac
     double np[3];
     R nd[3];
     helix_bz<R>(rn, sB, s, t.pos, t.dir, np, nd);
-    const R inv = R(1) / M<R>::sqrt(nd[0] * nd[0] + nd[1] * nd[1] + nd[2] * nd[2]);
+    R n2;
+    if constexpr (sizeof(R) == 4)
+      n2 = __fmaf_rn(nd[2], nd[2], __fmaf_rn(nd[1], nd[1], __fmul_rn(nd[0], nd[0])));
+    else
+      n2 = nd[0] * nd[0] + nd[1] * nd[1] + nd[2] * nd[2];
+    const R inv = R(1) / M<R>::sqrt(n2);
     for (int k = 0; k < 3; ++k) {
       t.pos[k] = np[k];
       t.dir[k] = nd[k] * inv;
