@@ -558,7 +558,7 @@ template <class R> struct Secs {
 __device__ __forceinline__ void sincos_t(float x, float *s, float *c) { sincosf(x, s, c); }
 __device__ __forceinline__ void sincos_t(double x, double *s, double *c) { ::sincos(x, s, c); }
 
-template <class T>
+template <class T, bool FUSED>
 __device__ __forceinline__ void helix_bz(T rn, T sB, double s, const double pos[3], const T dir[3], double np[3],
                                          T nd[3])
 {
@@ -567,9 +567,11 @@ __device__ __forceinline__ void helix_bz(T rn, T sB, double s, const double pos[
   sincos_t(T(0.5) * phi, &sh, &ch);
   const T sinp = T(2) * sh * ch, cm1 = T(-2) * sh * sh, cosp = T(1) + cm1;
   np[2] = pos[2] + s * (double)dir[2];
-  // FP32: which product of a sum is fused is written out; left open it differed
-  // from kernel to kernel, and a float's last bit is another track
-  if constexpr (sizeof(T) == 4) {
+  // FUSED (the FP32 kernels of the analytic navigator): which product of a sum is
+  // fused is written out; left open it differed from one form of their loop to
+  // another, and a float's last bit is another track.  The volume tree's kernels
+  // fuse others, the same in each form.
+  if constexpr (FUSED) {
     const float P = __fmul_rn(sinp, dir[0]), Q = __fmul_rn(sinp, dir[1]);
     np[0] = pos[0] + (double)(rn * __fmaf_rn(__fmul_rn(cm1, dir[1]), sB, -P));
     np[1] = pos[1] + (double)(rn * __fmaf_rn(__fmul_rn(-cm1, dir[0]), sB, -Q));
@@ -1174,9 +1176,10 @@ __device__ __forceinline__ bool field_substep(const Data &d, const Geom &g, Trac
     const R rn = p / (R(kB2C_mm) * charge * absB);
     double np[3];
     R nd[3];
-    helix_bz<R>(rn, sB, s, t.pos, t.dir, np, nd);
+    constexpr bool kFused = sizeof(R) == 4 && (K & kKindCsg) == 0;
+    helix_bz<R, kFused>(rn, sB, s, t.pos, t.dir, np, nd);
     R n2;
-    if constexpr (sizeof(R) == 4)
+    if constexpr (kFused)
       n2 = __fmaf_rn(nd[2], nd[2], __fmaf_rn(nd[1], nd[1], __fmul_rn(nd[0], nd[0])));
     else
       n2 = nd[0] * nd[0] + nd[1] * nd[1] + nd[2] * nd[2];
