@@ -131,6 +131,7 @@ _SIGS = {
     "gx_ioni_along_gpil": (I, [P, I, I, P, P, P, I, P]),
     "gx_ioni_along_doit": (I, [P, I, I, P, P, P, P, I, P]),
     "gx_helix_dostep": (I, [PD, D, I] + [P] * 15 + [P]),
+    "gx_helix_dostep_xyz": (I, [PD, D, I] + [P] * 7 + [P]),
     "gx_math_eval": (I, [I, I, I, P, P, P, P]),
     "gx_gpil": (I, [P, C.POINTER(TransportConfig), C.POINTER(TrackSoAStruct), P]),
     "gx_propagate": (I, [P, C.POINTER(TransportConfig), C.POINTER(TrackSoAStruct), P]),

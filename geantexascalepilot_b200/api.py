@@ -302,11 +302,11 @@ class ConstFieldHelixStepper:
         p = _dev(momentum, torch.float64)
         s = _dev(step, torch.float64)
         n = q.numel()
-        cols = [pos[:, k].contiguous() for k in range(3)] + [d[:, k].contiguous() for k in range(3)]
-        outs = [torch.empty(n, dtype=torch.float64, device="cuda") for _ in range(6)]
-        check(lib.gx_helix_dostep(self.B, self.kB2C, n, *[_ptr(c) for c in cols], _ptr(q), _ptr(p), _ptr(s),
-                                  *[_ptr(o) for o in outs], _stream()))
-        return torch.stack(outs[:3], 1), torch.stack(outs[3:], 1)
+        newpos, newdir = torch.empty((n, 3), dtype=torch.float64, device="cuda"), torch.empty(
+            (n, 3), dtype=torch.float64, device="cuda")
+        check(lib.gx_helix_dostep_xyz(self.B, self.kB2C, n, _ptr(pos), _ptr(d), _ptr(q), _ptr(p), _ptr(s),
+                                      _ptr(newpos), _ptr(newdir), _stream()))
+        return newpos, newdir
 
 
 # ------------------------------------------------------- tracks in SoA form

@@ -308,9 +308,11 @@ __global__ void k_along_doit(const Data *__restrict__ d, int mode, int charge, c
 }
 
 // ----------------------------------------------------------------- helix
+// stride: between the tracks' values of a component (1: a plane each, 3: xyz
+// interleaved)
 struct HelixArgs {
   double B[3], kB2C;
-  int n;
+  int n, stride;
   const double *px, *py, *pz, *dx, *dy, *dz, *q, *p, *s;
   double *npx, *npy, *npz, *ndx, *ndy, *ndz;
 };
@@ -319,14 +321,15 @@ __global__ void k_helix(HelixArgs a)
 {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
-  double pos[3] = {a.px[i], a.py[i], a.pz[i]}, dir[3] = {a.dx[i], a.dy[i], a.dz[i]}, np[3], nd[3];
+  const long long j = (long long)i * a.stride;
+  double pos[3] = {a.px[j], a.py[j], a.pz[j]}, dir[3] = {a.dx[j], a.dy[j], a.dz[j]}, np[3], nd[3];
   helix_dostep(a.kB2C, a.B, pos, dir, a.q[i], a.p[i], a.s[i], np, nd);
-  a.npx[i] = np[0];
-  a.npy[i] = np[1];
-  a.npz[i] = np[2];
-  a.ndx[i] = nd[0];
-  a.ndy[i] = nd[1];
-  a.ndz[i] = nd[2];
+  a.npx[j] = np[0];
+  a.npy[j] = np[1];
+  a.npz[j] = np[2];
+  a.ndx[j] = nd[0];
+  a.ndy[j] = nd[1];
+  a.ndz[j] = nd[2];
 }
 
 static int check_launch(const char *what)
@@ -581,8 +584,20 @@ int gx_helix_dostep(const double B[3], double kB2C, int n, const double *d_posx,
                     gx_stream_t s)
 {
   if (!B || n < 0) return set_error(GX_ERR_ARG, "gx_helix_dostep: bad args");
-  HelixArgs a = {{B[0], B[1], B[2]}, kB2C, n, d_posx, d_posy, d_posz, d_dirx, d_diry, d_dirz, d_charge, d_momentum,
+  HelixArgs a = {{B[0], B[1], B[2]}, kB2C, n, 1, d_posx, d_posy, d_posz, d_dirx, d_diry, d_dirz, d_charge, d_momentum,
                  d_step, d_newposx, d_newposy, d_newposz, d_newdirx, d_newdiry, d_newdirz};
+  if (n > 0) k_helix<<<grid_for(n), kBlock, 0, stream_of(s)>>>(a);
+  return check_launch("k_helix");
+}
+
+int gx_helix_dostep_xyz(const double B[3], double kB2C, int n, const double *d_pos, const double *d_dir,
+                        const double *d_charge, const double *d_momentum, const double *d_step, double *d_newpos,
+                        double *d_newdir, gx_stream_t s)
+{
+  if (!B || n < 0 || (n > 0 && (!d_pos || !d_dir || !d_charge || !d_momentum || !d_step || !d_newpos || !d_newdir)))
+    return set_error(GX_ERR_ARG, "gx_helix_dostep_xyz: bad args");
+  HelixArgs a = {{B[0], B[1], B[2]}, kB2C, n, 3, d_pos, d_pos + 1, d_pos + 2, d_dir, d_dir + 1, d_dir + 2, d_charge,
+                 d_momentum, d_step, d_newpos, d_newpos + 1, d_newpos + 2, d_newdir, d_newdir + 1, d_newdir + 2};
   if (n > 0) k_helix<<<grid_for(n), kBlock, 0, stream_of(s)>>>(a);
   return check_launch("k_helix");
 }

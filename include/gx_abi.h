@@ -202,6 +202,12 @@ int gx_helix_dostep(const double B[3], double kB2C, int n, const double *d_posx,
                     double *d_newposy, double *d_newposz, double *d_newdirx, double *d_newdiry,
                     double *d_newdirz, gx_stream_t s);
 
+/* The same with positions and directions interleaved (xyz of each track, n x 3),
+ * as a caller that keeps vectors has them: no planes to copy out and back. */
+int gx_helix_dostep_xyz(const double B[3], double kB2C, int n, const double *d_pos, const double *d_dir,
+                        const double *d_charge, const double *d_momentum, const double *d_step, double *d_newpos,
+                        double *d_newdir, gx_stream_t s);
+
 /* ------------------------------------------------------- CSG geometry */
 /* A volume tree for transport geometry 2, built with the calls a VecGeom
  * detector construction makes (the reference navigates VecGeom,
