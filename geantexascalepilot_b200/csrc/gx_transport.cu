@@ -818,10 +818,10 @@ __global__ void k_refill_done(Ctl *ctl)
   ctl->take_prim = 0;
 }
 
-__global__ void k_count_new_tracks(Ctl *ctl)
+// Tracks of a run: the primaries, and every secondary once.
+inline long long total_tracks(const Ctl &c)
 {
-  // every secondary becomes a track exactly once
-  ctl->stat[S_TRACKS] += ctl->stat[S_SEC0] + ctl->stat[S_SEC1] + ctl->stat[S_SEC2];
+  return (long long)(c.stat[S_TRACKS] + c.stat[S_SEC0] + c.stat[S_SEC1] + c.stat[S_SEC2]);
 }
 
 // ------------------------------------------------------------------ engine
@@ -1425,6 +1425,7 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
     }
     for (;;) {
       if ((err = cudaGraphLaunch(E->graph, s)) != cudaSuccess) return cuda_error(err, "graph launch");
+      cudaEventRecord(t1, s);
       cudaMemcpyAsync(E->h_ctl, E->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
       if ((err = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(err, "transport graph");
       iters = E->h_ctl->iterations;
@@ -1437,7 +1438,6 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
     k_fold_touchables<<<(int)std::min<long long>((nt + 255) / 256, 4096), 256, 0, s>>>(
         E->vtally, C->csg_score, C->csg_n, C->csg_nscore, nt, d_edep);
   }
-  k_count_new_tracks<<<1, 1, 0, s>>>(E->ctl);
   if (tout) {
     // the tracks still alive: carry out the refill plan the last iteration
     // made (deferred tracks back into the stores, the next primaries in), then
@@ -1463,9 +1463,12 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
                                                                                         np, E->ctl, *tout);
     }
   }
-  cudaEventRecord(t1, s);
-  cudaMemcpyAsync(E->h_ctl, E->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
-  if ((err = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(err, "transport end");
+  // the graph's last look at the counters is the end, unless something followed it
+  if (!batched || cfg->profile || max_iter > 0 || cfg->geometry == 2 || tout) {
+    cudaEventRecord(t1, s);
+    cudaMemcpyAsync(E->h_ctl, E->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
+    if ((err = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(err, "transport end");
+  }
   float ms = 0;
   cudaEventElapsedTime(&ms, t0, t1);
   cudaEventDestroy(t0);
@@ -1474,7 +1477,7 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
   if (stats) {
     stats->steps = (long long)c.stat[S_STEPS];
     stats->substeps = (long long)c.stat[S_SUBSTEPS];
-    stats->tracks = (long long)c.stat[S_TRACKS];
+    stats->tracks = total_tracks(c);
     for (int q = 0; q < 3; ++q) stats->secondaries[q] = (long long)c.stat[S_SEC0 + q];
     stats->n_pair = (long long)c.stat[S_PAIR];
     stats->n_annih = (long long)c.stat[S_ANNIH];
@@ -2200,7 +2203,6 @@ extern "C" int gx_transport_run_noalloc(gx_ctx *ctx, const gx_transport_config *
     if (hc.in_flight == 0 && hc.pending == 0) break;
     if (iters > 2000000LL) return set_error(GX_ERR_ITERCAP, "gx_transport_run_noalloc: iteration cap");
   }
-  k_count_new_tracks<<<1, 1, 0, s>>>(ctl);
   if ((err = cudaMemcpyAsync(&hc, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
       (err = cudaStreamSynchronize(s)) != cudaSuccess)
     return cuda_error(err, "gx_transport_run_noalloc: end");
@@ -2208,7 +2210,7 @@ extern "C" int gx_transport_run_noalloc(gx_ctx *ctx, const gx_transport_config *
     std::memset(stats, 0, sizeof(*stats));
     stats->steps = (long long)hc.stat[S_STEPS];
     stats->substeps = (long long)hc.stat[S_SUBSTEPS];
-    stats->tracks = (long long)hc.stat[S_TRACKS];
+    stats->tracks = total_tracks(hc);
     for (int q = 0; q < 3; ++q) stats->secondaries[q] = (long long)hc.stat[S_SEC0 + q];
     stats->n_pair = (long long)hc.stat[S_PAIR];
     stats->n_annih = (long long)hc.stat[S_ANNIH];
