@@ -838,8 +838,8 @@ __device__ __noinline__ double3 msc_displacement(const Geom &g, int vol, double 
 // the volume and deposits all of e there, whatever the direction (step_gpil,
 // field_substep: safety above the remaining length; along_loss: step >= range).
 // The margin is far above the move's rounding and the navigator's snap distance.
-// range: the step.
-template <class R>
+// range: the step.  S: the solids of the volume tree (0: the analytic volumes).
+template <class R, int S>
 __device__ __forceinline__ bool stops_at_once(const Data &d, const Geom &g, int vol, const double *pos, int mat, R e,
                                               R &range)
 {
@@ -847,7 +847,13 @@ __device__ __forceinline__ bool stops_at_once(const Data &d, const Geom &g, int 
   range = range_limit<R>(d, 1, mat, e, raw);
   const R cut = (R)d.cut_length[1][mat], finR = (R(10.0) < cut) ? R(10.0) : cut;
   if (e < R(kMinE)) raw *= e / R(kMinE);
-  return raw <= finR && safety(g, vol, pos) > 1.0001 * (double)range + 2e-6;
+  if (!(raw <= finR)) return false;
+  double saf;
+  if constexpr (S != 0)
+    saf = csg_safety<S>(g.csg, vol, pos);
+  else
+    saf = safety(g, vol, pos);
+  return saf > 1.0001 * (double)range + 2e-6;
 }
 #endif
 

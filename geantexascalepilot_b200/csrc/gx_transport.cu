@@ -397,14 +397,15 @@ template <class R, int PT, int K> __global__ void __launch_bounds__(1024, 1) k_t
 #ifndef GX_PARITY
 // Electrons that stops_at_once() finds to end in the volume they are created in never become
 // records: about half of all e- steps are the only step of a photo-electron or a
-// Compton electron, and it leaves nothing but its deposit and its counts.  In
-// the layered or box geometry, without multiple scattering, and with enough of
+// Compton electron, and it leaves nothing but its deposit and its counts.
+// Without multiple scattering, and with enough of
 // them (n, the interactions of a launch) that throughput counts: 20000 showers
-// 128.9 to 123.7 ms, 256 events 169.8 to 163.7, but two electrons 3.06 to 3.16,
-// where the looking is latency on the way to the next iteration.
+// 128.9 to 123.7 ms, 256 events 169.8 to 163.7, 1001 through the volume tree 30.4
+// to 29.1, but two electrons 3.06 to 3.16, where the looking is latency on the way
+// to the next iteration.
 __device__ __forceinline__ bool local_stops(const Geom &g, long long n)
 {
-  return !g.msc && g.geometry != 2 && !g.charged_local && n >= 1024;
+  return !g.msc && !g.charged_local && n >= 1024;
 }
 
 template <class R> __device__ __forceinline__ void book_stop(const Geom &g, const Track<R> &t, R e, Local &L)
@@ -419,14 +420,15 @@ template <class R> __device__ __forceinline__ void book_stop(const Geom &g, cons
 // before (no cross section at its energy): its energy and the shell's are
 // deposited, and neither its direction nor its stream is sampled, since nothing
 // is left that would use them.
-template <class R> __device__ __forceinline__ bool photo_electron_stops(const Data &d, const Geom &g, Track<R> &t, Local &L)
+template <class R, int S>
+__device__ __forceinline__ bool photo_electron_stops(const Data &d, const Geom &g, Track<R> &t, Local &L)
 {
   const int mat = vol_material(g, t.vol);
   const R e = (R)photo_electron_energy(d, (int)d.mat_Z[mat], (double)t.E, 1);
   if (!(e > R(0)) || (double)e > d.vec[GX_Lambda_eIoni_em][mat].emin || (double)e > d.vec[GX_Lambda_eBrem_em][mat].emin)
     return false;
   R range;
-  if (!stops_at_once<R>(d, g, t.vol, t.pos, mat, e, range)) return false;
+  if (!stops_at_once<R, S>(d, g, t.vol, t.pos, mat, e, range)) return false;
   L.deposit(t.event, t.vol, (double)(t.E - e));
   book_stop(g, t, e, L);
   t.E = R(0);
@@ -436,7 +438,7 @@ template <class R> __device__ __forceinline__ bool photo_electron_stops(const Da
 // emit_tracks for a Compton scattering or photo-electric absorption (at most one
 // electron, in the batched engine's three stores): the electron is booked on the
 // spot when `local` and it stops at once before any interaction.
-template <class R>
+template <class R, int S>
 __device__ __forceinline__ void emit_electron(const Args<R> &a, Ctl *ctl, int par, bool active, bool alive, Track<R> &t,
                                               const Secs<R> &sec, bool local, Local &L)
 {
@@ -460,7 +462,7 @@ __device__ __forceinline__ void emit_electron(const Args<R> &a, Ctl *ctl, int pa
       c.set_rng(cr);
       const int mat = vol_material(a.g, c.vol);
       R range;
-      if (local && stops_at_once<R>(*a.d, a.g, c.vol, c.pos, mat, c.E, range)) {
+      if (local && stops_at_once<R, S>(*a.d, a.g, c.vol, c.pos, mat, c.E, range)) {
         // as step_gpil chooses: a process comes first unless its length is above the range
         R xs[3];
         cross_sections<R>(*a.d, 1, mat, c.E, xs);
@@ -489,7 +491,10 @@ __device__ __forceinline__ void emit_electron(const Args<R> &a, Ctl *ctl, int pa
 // Post-step interaction of process PROC for the buffered tracks of type PT:
 // one model per kernel, so a warp runs one sampling algorithm; survivor and
 // secondaries go to the next stores.
-template <class R, int PT, int PROC> __device__ __forceinline__ void interact_body(const Args<R> *__restrict__ A)
+// S: the solids of the volume tree, in the kernels that look at the geometry (0:
+// the analytic volumes).
+template <class R, int PT, int PROC, int S>
+__device__ __forceinline__ void interact_body(const Args<R> *__restrict__ A)
 {
   extern __shared__ double sm_edep[];
   __shared__ unsigned long long sm_stat[kNStat];
@@ -524,7 +529,7 @@ template <class R, int PT, int PROC> __device__ __forceinline__ void interact_bo
       L.st[S_READ0 + PT]++;
       bool sample = true;
 #ifndef GX_PARITY
-      if (PT == 0 && PROC == 2 && local) sample = !photo_electron_stops(d, a.g, t, L);
+      if (PT == 0 && PROC == 2 && local) sample = !photo_electron_stops<R, S>(d, a.g, t, L);
 #endif
       if (sample) {
         run_model(d, a.g, t, PROC, sec, L);
@@ -533,7 +538,7 @@ template <class R, int PT, int PROC> __device__ __forceinline__ void interact_bo
     }
 #ifndef GX_PARITY
     if constexpr (PT == 0 && PROC != 1)
-      emit_electron(a, ctl, par, active, alive, t, sec, local, L);
+      emit_electron<R, S>(a, ctl, par, active, alive, t, sec, local, L);
     else
 #endif
       emit_tracks<R, PT>(a, ctl, par, active, alive, t, sec, L);
@@ -542,15 +547,15 @@ template <class R, int PT, int PROC> __device__ __forceinline__ void interact_bo
   GX_TL_END();
 }
 
-template <class R, int PT, int PROC>
+template <class R, int PT, int PROC, int S>
 __global__ void __launch_bounds__(256, kMinBlocks<R>) __maxnreg__((kMaxRegs<R, 0>)) k_interact(const Args<R> *__restrict__ A)
 {
-  interact_body<R, PT, PROC>(A);
+  interact_body<R, PT, PROC, S>(A);
 }
 template <class R, int PT, int PROC>
 __global__ void __launch_bounds__(1024, 1) k_interact_wide(const Args<R> *__restrict__ A)
 {
-  interact_body<R, PT, PROC>(A);
+  interact_body<R, PT, PROC, 0>(A);
 }
 
 // End of an iteration: the refill that opened it is booked, the next stores
@@ -959,7 +964,13 @@ template <class R, int PT, int PROC> static void (*interact_for(const Launch<R> 
 #ifndef GX_PARITY
   if (L.block > 256) return k_interact_wide<R, PT, PROC>;
 #endif
-  return k_interact<R, PT, PROC>;
+#ifndef GX_PARITY
+  if constexpr (PT == 0 && PROC != 1)
+    if (L.a.g.geometry == 2)
+      return sizeof(R) == 4 && L.a.g.csg.solids == kSolidsBox ? k_interact<R, PT, PROC, kSolidsBox>
+                                                              : k_interact<R, PT, PROC, kSolidsAll>;
+#endif
+  return k_interact<R, PT, PROC, 0>;
 }
 
 // One type's interaction kernels (gamma 3 processes, e- 2, e+ 3): one after

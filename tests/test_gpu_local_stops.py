@@ -19,14 +19,17 @@ def dm():
 
 
 @pytest.mark.parametrize("Bz", [0.0, 4.0])
-@pytest.mark.parametrize("geometry,charged_local", [("layers", 0), ("box", 0), ("box", 1)])
+@pytest.mark.parametrize("geometry,charged_local", [("layers", 0), ("box", 0), ("box", 1), ("tree", 0)])
 @pytest.mark.parametrize("n,energy", [(3, 50.0), (4000, 2.0)])
 def test_batched_engine_equals_the_plain_loop(dm, n, energy, geometry, charged_local, Bz):
     import geantexascalepilot_b200 as g
     from geantexascalepilot_b200 import configs
     cfg, _, nvol = configs.c1(1)
-    if geometry == "layers":
+    if geometry != "box":
         cfg, _, nvol = configs.c2(1)
+    if geometry == "tree":
+        nvol = dm.load_geometry(g.geometry.calorimeter(axis=cfg.axis))
+        cfg.geometry = 2
     cfg.charged_local, cfg.Bz = charged_local, Bz
     rng = np.random.default_rng(5)
     pos = rng.uniform(-40.0, 40.0, (n, 3)) + (np.array([0.0, 0.0, 50.0]) if geometry == "box" else 0.0)
