@@ -313,8 +313,9 @@ def main():
         for _ in range(steps):
             st = one(precision, engine, parity=parity, c=c, tens=tens, events=events, out=out)
             n_steps += st["steps"]
-            # per iteration: refill, refill_done, 3 transport, 8 interaction, finish; plain loop: 4
-            launches += (14 if engine == 1 else 4) * (st["iterations"] + 1) + 3
+            # per iteration: refill, 3 transport, 8 interaction, finish; plain loop: refill, step,
+            # finish; before the first one: energy prefix sums and the refill plan
+            launches += (13 if engine == 1 else 3) * st["iterations"] + 2
         ev1.record()
         barrier()
         ms = ev0.elapsed_time(ev1)
@@ -333,7 +334,7 @@ def main():
         trials = gx.autotune(dm, cfg, dev["t"], dev["E"], dev["p"], dev["d"], nvol=nvol, repeats=2)
         tuned = {"best": trials[0], "trials": len(trials),
                  "default": next((t for t in trials if t["block_size"] == 128 and t["blocks_per_sm"] == 5
-                                  and t["steps_per_launch"] == 16 and t["graph_iters"] == 16
+                                  and t["steps_per_launch"] == 0 and t["graph_iters"] == 0
                                   and t["wave_energy"] == 0), None)}
 
     # headline: FP32-mixed, batched engine, primaries resident in HBM
@@ -350,8 +351,8 @@ def main():
            "primaries_per_s": world * nprim * args.steps / (ms / 1e3),
            "stats": {k: st32[k] for k in ("steps", "substeps", "tracks", "iterations", "peak_in_flight", "errors")},
            "launch": {"block": cfg.block_size or 128, "blocks_per_sm": cfg.blocks_per_sm or 5,
-                      "steps_per_launch": cfg.steps_per_launch or 16,
-                      "graph_iters": cfg.graph_iters or 16}}
+                      "steps_per_launch": cfg.steps_per_launch or "by type and population",
+                      "graph_iters": cfg.graph_iters or "repeats on the device"}}
     if tuned:
         out["autotune"] = tuned
 

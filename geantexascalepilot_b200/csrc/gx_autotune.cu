@@ -60,7 +60,7 @@ extern "C" int gx_transport_autotune(gx_ctx *ctx, gx_transport_config *cfg, int 
   Trial best = {base.block_size > 0 ? base.block_size : default_block(1),
                 base.blocks_per_sm > 0 ? base.blocks_per_sm : default_blocks_per_sm(base),
                 base.steps_per_launch > 0 ? base.steps_per_launch : 0, // 0: the engine's own choice
-                base.graph_iters > 0 ? base.graph_iters : 16,
+                base.graph_iters > 0 ? base.graph_iters : 0, // 0: the graph repeats by itself
                 base.refill_below > 0 ? base.refill_below : cap / 2, base.wave_energy,
                 base.interaction_interval > 0 ? base.interaction_interval : 1,
                 base.fetch_min_by_type[0] > 0 ? base.fetch_min_by_type[0] : default_fetch_min(base, 0)};

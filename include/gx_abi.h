@@ -341,7 +341,8 @@ typedef struct {
   long long transport_read[3];    /* track records read */
   long long transport_written[3]; /* records written: survivors and interacting tracks */
   long long transport_queued[3];  /* of those, records written to the interaction buffers */
-  long long transport_steps[3];   /* steps completed in the transport kernel */
+  long long transport_steps[3];   /* steps completed in the transport kernel; e-: and the only steps of those that
+                              the interaction kernels book where they stop */
 } gx_transport_stats;
 
 void gx_transport_config_default(gx_transport_config *cfg);
@@ -553,8 +554,8 @@ int gx_transport_tracks(gx_ctx *ctx, const gx_transport_config *cfg, const gx_tr
  * candidate: block size {64, 128, 256, 512, 1024} (512 and 1024 with the
  * uniform field, layered geometry and no multiple scattering, at most 4096
  * threads per SM) x resident blocks per SM {1, 2, 4, 5, 6, 8}, then steps per track
- * and transport launch {1, 16, 64, 1024}, then iterations per CUDA-graph
- * launch {4, 8, 32, 64}, then the refill threshold {1/8, 1/4, 3/4 of the
+ * and transport launch {1, 16, 64, 1024} and iterations per CUDA-graph launch
+ * {4, 8, 32, 64} beside the engine's own choice (0), then the refill threshold {1/8, 1/4, 3/4 of the
  * capacity}, then the primary energy per injection wave {1/4, 1/2, 2 x the
  * default}, then the compaction interval (interaction_interval) {2, 4, 8},
  * then the photon kernel's fetch threshold (fetch_min_by_type[0]) {1, 8, 16,
