@@ -1537,6 +1537,7 @@ struct StageArgs {
   gx_track_soa t, sec;
   double *edep;
   double *escaped;
+  int sorted; // the blocks work in the order of stage_track
 };
 
 __device__ __forceinline__ void soa_load(const gx_track_soa &s, int i, Track<double> &t)
@@ -1612,12 +1613,13 @@ __device__ __forceinline__ void stage_local(Local &L, const StageArgs &a)
 
 // The tracks of a stage's block in the order of `key` (0 .. 15, -1: nothing to
 // do): the thread's track, -1 for none.  A batch in flight mixes particle types
-// and processes, whose code a warp would run one after another; sorted within a
-// block of kStageBlock, most warps run one of them (100003 tracks: gx_post_step
-// 112 us in the batch's order, 48 in this; gx_propagate 72 and 63; gx_gpil and
-// gx_along_step, where the types share most of the code, gain nothing and keep
-// the batch's order).  Every thread of the block calls it.
-constexpr int kStageBlock = 256;
+// and processes, whose models a warp of gx_post_step would run one after another;
+// sorted within a block of kStageBlock, most warps run one of them (400000 tracks
+// 508 us in the batch's order, 196 in this; 100003 99 and 51; 32000 53 and 39;
+// 16000 39 and 35; 8000 31 and 35, so from kStageSortFrom on).  The other stages,
+// whose types share most of the code, gain nothing by it.  Every thread of the
+// block calls it.
+constexpr int kStageBlock = 256, kStageSortFrom = 16384;
 __device__ __forceinline__ int stage_track(int key)
 {
   __shared__ int first[17], order[kStageBlock];
@@ -1630,13 +1632,13 @@ __device__ __forceinline__ int stage_track(int key)
   if (t == 0)
     for (int k = 1; k < 17; ++k) first[k] += first[k - 1];
   __syncthreads();
-  if (key >= 0) order[first[key] + rank] = blockIdx.x * kStageBlock + t;
+  if (key >= 0) order[first[key] + rank] = blockIdx.x * blockDim.x + t;
   __syncthreads();
   return order[t];
 }
-template <int K> __global__ void __launch_bounds__(kStageBlock) k_stage_gpil(StageArgs a)
+template <int K> __global__ void __launch_bounds__(128) k_stage_gpil(StageArgs a)
 {
-  const int i = blockIdx.x * kStageBlock + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.t.n || a.t.status[i] != GX_TRACK_ALIVE) return;
   Track<double> t;
   soa_load(a.t, i, t);
@@ -1659,11 +1661,10 @@ template <int K> __global__ void __launch_bounds__(kStageBlock) k_stage_gpil(Sta
   a.t.snext[i] = fmin(nav_distance<K>(a.g, t.vol, t.pos, t.dir, ps, plane), ps);
 }
 
-template <int K> __global__ void __launch_bounds__(kStageBlock) k_stage_propagate(StageArgs a)
+template <int K> __global__ void __launch_bounds__(128) k_stage_propagate(StageArgs a)
 {
-  const int own = blockIdx.x * kStageBlock + threadIdx.x;
-  const int i = stage_track(own < a.t.n && a.t.status[own] == GX_TRACK_ALIVE ? min(max(a.t.type[own], 0), 3) : -1);
-  if (i < 0) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.t.n || a.t.status[i] != GX_TRACK_ALIVE) return;
   Track<double> t;
   soa_load(a.t, i, t);
   StepCtx<double> c;
@@ -1679,9 +1680,9 @@ template <int K> __global__ void __launch_bounds__(kStageBlock) k_stage_propagat
   a.t.next_volume[i] = c.crossed ? c.newvol : t.vol;
 }
 
-template <int K> __global__ void __launch_bounds__(kStageBlock) k_stage_along(StageArgs a)
+template <int K> __global__ void __launch_bounds__(128) k_stage_along(StageArgs a)
 {
-  const int i = blockIdx.x * kStageBlock + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.t.n || a.t.status[i] != GX_TRACK_ALIVE) return;
   Track<double> t;
   soa_load(a.t, i, t);
@@ -1704,11 +1705,11 @@ template <int K> __global__ void __launch_bounds__(kStageBlock) k_stage_along(St
 
 template <int K> __global__ void __launch_bounds__(kStageBlock) k_stage_post(StageArgs a)
 {
-  const int own = blockIdx.x * kStageBlock + threadIdx.x;
+  const int own = blockIdx.x * blockDim.x + threadIdx.x;
   int key = -1; // interacting: by type and process; 15: only the secondaries' slots to clear
   if (own < a.t.n)
     key = a.t.status[own] == GX_TRACK_INTERACT ? min(max(a.t.type[own] * 3 + a.t.process[own], 0), 14) : 15;
-  const int i = stage_track(key);
+  const int i = a.sorted ? stage_track(key) : (key >= 0 ? own : -1);
   if (i < 0) return;
   int nsec = 0;
   if (a.t.status[i] == GX_TRACK_INTERACT) {
@@ -1777,13 +1778,14 @@ int run_stage(int stage, Ctx *C, const gx_transport_config *cfg, gx_track_soa *t
   a.edep = d_edep;
   a.escaped = C->stage_scratch;
   if (t->n <= 0) return GX_OK;
-  const int grid = (t->n + kStageBlock - 1) / kStageBlock;
+  a.sorted = stage == 3 && t->n >= kStageSortFrom;
+  const int block = a.sorted ? kStageBlock : 128, grid = (t->n + block - 1) / block;
   const bool fm = cfg->field_map != 0;
   switch (stage) {
-  case 0: (fm ? k_stage_gpil<kKindFieldMap> : k_stage_gpil<0>)<<<grid, kStageBlock, 0, s>>>(a); break;
-  case 1: (fm ? k_stage_propagate<kKindFieldMap> : k_stage_propagate<0>)<<<grid, kStageBlock, 0, s>>>(a); break;
-  case 2: (fm ? k_stage_along<kKindFieldMap> : k_stage_along<0>)<<<grid, kStageBlock, 0, s>>>(a); break;
-  default: (fm ? k_stage_post<kKindFieldMap> : k_stage_post<0>)<<<grid, kStageBlock, 0, s>>>(a); break;
+  case 0: (fm ? k_stage_gpil<kKindFieldMap> : k_stage_gpil<0>)<<<grid, block, 0, s>>>(a); break;
+  case 1: (fm ? k_stage_propagate<kKindFieldMap> : k_stage_propagate<0>)<<<grid, block, 0, s>>>(a); break;
+  case 2: (fm ? k_stage_along<kKindFieldMap> : k_stage_along<0>)<<<grid, block, 0, s>>>(a); break;
+  default: (fm ? k_stage_post<kKindFieldMap> : k_stage_post<0>)<<<grid, block, 0, s>>>(a); break;
   }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GX_OK : cuda_error(e, "gx stage launch");

@@ -1,6 +1,7 @@
-"""The stage calls work on a batch in an order of their own (by particle type and
-process within a block of 256): a batch gives each track what it gets alone, at
-the edges of the blocks, and slots without an interaction are cleared."""
+"""gx_post_step works on a batch of 16384 tracks or more in an order of its own (by
+particle type and process within a block of 256): a batch gives each track what it
+gets alone, at the edges of the blocks and of that rule, and slots without an
+interaction are cleared."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -21,12 +22,12 @@ def _batch(g, cfg, index):
     import numpy as np
     k = np.asarray(index)
     rng = np.random.default_rng(11)
-    d = rng.normal(size=(2048, 3))
-    pos = rng.uniform(-190.0, 190.0, (2048, 3))
-    E = 10.0 ** rng.uniform(-1.0, 4.0, 2048)
+    d = rng.normal(size=(20000, 3))
+    pos = rng.uniform(-190.0, 190.0, (20000, 3))
+    E = 10.0 ** rng.uniform(-1.0, 4.0, 20000)
     d /= np.linalg.norm(d, axis=1)[:, None]
     t = g.TrackSoA.from_primaries(cfg, k % 3, E[k], pos[k], d[k])
-    st = g.MRG32k3a.substreams(list(cfg.seed), 0, 2048)
+    st = g.MRG32k3a.substreams(list(cfg.seed), 0, 20000)
     t.rng.view(6, t.capacity)[:, :len(k)] = st[:, k]
     return t
 
@@ -45,7 +46,7 @@ def _step(g, dm, cfg, t):
             [getattr(sec, f).cpu() for f in FIELDS] + [sec.rng.view(6, sec.capacity).cpu()])
 
 
-@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 1025])
+@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 1025, 16383, 16384, 16641])
 def test_a_batch_gives_each_track_what_it_gets_alone(dm, n):
     import numpy as np
     import torch
