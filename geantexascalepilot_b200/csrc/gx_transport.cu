@@ -599,6 +599,8 @@ __device__ void finish_iteration(Ctl *ctl, long long cap0, long long cap1, long 
   for (int q = 0; q < nstores; ++q) {
     long long room = cap[q] - ctl->count[np][q];
     long long take = 0;
+    // all of the stack is pending, also what is taken now: it is in no store yet
+    pend += ctl->stack_count[q];
     if (budget > 0) take = min(min(ctl->stack_count[q], room), budget);
     // reserve the slots now: deferred tracks land at the end of the store,
     // primaries are appended after them by the refill kernel
@@ -608,7 +610,6 @@ __device__ void finish_iteration(Ctl *ctl, long long cap0, long long cap1, long 
     ctl->stack_count[q] -= take;
     ctl->stack_src[q] = ctl->stack_count[q];
     budget -= take;
-    pend += ctl->stack_count[q];
   }
   // primaries: a shower's population peaks in proportion to its energy, long
   // after it is injected, so primaries are injected only while the energy the
