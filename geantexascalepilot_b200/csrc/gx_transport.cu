@@ -644,9 +644,11 @@ __device__ void finish_iteration(Ctl *ctl, long long cap0, long long cap1, long 
 // block reads and writes together: word by word from L2 it took 4.2 us of every
 // iteration, and the booking of the refill was a launch of its own.
 constexpr int kFinishBlock = 128;
-// loop: the conditional node of the graph this runs in (0: none), which repeats
-// its `batch` iterations while tracks are left, until a multiple of kLoopIters
-// is reached (the host then launches it again).
+// batch > 0: the last of the `batch` iterations in the body of the conditional
+// node `loop`, which repeats while tracks are left, until a multiple of kLoopIters
+// is reached (the host then launches it again).  Every pass of the body sets the
+// node's condition, whatever the handle's value (0 is not documented as invalid):
+// a pass that did not would leave it at its default and repeat for good.
 constexpr long long kLoopIters = 4096;
 __global__ void __launch_bounds__(kFinishBlock) k_finish(Ctl *ctl, long long cap0, long long cap1, long long cap2,
                                                          int nstores, int interacted, cudaGraphConditionalHandle loop, int batch)
@@ -659,7 +661,7 @@ __global__ void __launch_bounds__(kFinishBlock) k_finish(Ctl *ctl, long long cap
   __syncthreads();
   if (threadIdx.x == 0) {
     finish_iteration(&c, cap0, cap1, cap2, nstores, interacted);
-    if (loop)
+    if (batch > 0)
       cudaGraphSetConditional(loop, (c.in_flight || c.pending) &&
                                         c.iterations / kLoopIters == (c.iterations - batch) / kLoopIters);
   }
@@ -1075,7 +1077,7 @@ template <class R> static cudaError_t loop_graph(const Launch<R> &L, Engine *e, 
   if (err == cudaSuccess) {
     const int batch = (kLoopBatch + every - 1) / every * every;
     for (int k = 0; k < batch; ++k)
-      enqueue_iteration(L, e, cs, true, (k + 1) % every == 0, k + 1 == batch ? loop : 0, batch);
+      enqueue_iteration(L, e, cs, true, (k + 1) % every == 0, loop, k + 1 == batch ? batch : 0);
     cudaGraph_t body = nullptr;
     err = cudaStreamEndCapture(cs, &body);
   }
