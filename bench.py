@@ -511,7 +511,8 @@ def main():
     k = int(np.argmax(stp["transport_ms"]))
     launches_k = max(1, stp["step_launches"][k])
     k_ms = stp["transport_ms"][k]
-    k_steps = stp["transport_steps"][k]
+    # the steps that the kernel makes: without the e- steps that the interaction kernels book
+    k_steps = stp["transport_steps"][k] - (stp["booked_steps"] if k == 1 else 0)
     k_records = stp["transport_read"][k] + stp["transport_written"][k]
     # algorithmic bytes: one read and one write of the track record per step
     # (a step reads and writes the state once); the kernel keeps a track in

@@ -45,17 +45,19 @@ struct Geom {
   CsgView csg; // geometry 2: the context's volume tree
 };
 
-constexpr int kNStat = 28;
+constexpr int kNStat = 29;
 // S_READ/S_WRITE: track records read and written by the step kernels of a
 // type other than its transport kernel (the interaction kernels, the plain
 // loop's fused kernel); S_TREAD/S_TWRITE: by its transport kernel (the host
 // reports the sums as the type's records read and written); S_TQUEUE: of the
 // transport kernel's writes, the records put in an interaction buffer (added
 // up by k_finish from the buffers' counters); S_TSTEP: steps completed in the
-// transport kernel of a type.
+// transport kernel of a type; S_BOOKED: steps of electrons that the interaction
+// kernels book where they stop.
 enum { S_STEPS, S_SUBSTEPS, S_TRACKS, S_SEC0, S_SEC1, S_SEC2, S_PAIR, S_ANNIH, S_ERR, S_OVERFLOW,
        S_READ0, S_READ1, S_READ2, S_WRITE0, S_WRITE1, S_WRITE2, S_TREAD0, S_TREAD1, S_TREAD2,
-       S_TWRITE0, S_TWRITE1, S_TWRITE2, S_TQUEUE0, S_TQUEUE1, S_TQUEUE2, S_TSTEP0, S_TSTEP1, S_TSTEP2 };
+       S_TWRITE0, S_TWRITE1, S_TWRITE2, S_TQUEUE0, S_TQUEUE1, S_TQUEUE2, S_TSTEP0, S_TSTEP1, S_TSTEP2,
+       S_BOOKED };
 
 struct Ctl {
   int parity;

@@ -543,7 +543,7 @@ __device__ __forceinline__ void interact_body(const Args<R> *__restrict__ A)
 #endif
       emit_tracks<R, PT>(a, ctl, par, active, alive, t, sec, L);
   }
-  tally_end(L, ctl, a.edep, sm_edep, sm_stat, sm_esc, &sm_err, S_TSTEP1);
+  tally_end(L, ctl, a.edep, sm_edep, sm_stat, sm_esc, &sm_err, S_BOOKED);
   GX_TL_END();
 }
 
@@ -1512,6 +1512,8 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
       stats->transport_queued[q] = (long long)c.stat[S_TQUEUE0 + q];
       stats->transport_steps[q] = (long long)c.stat[S_TSTEP0 + q];
     }
+    stats->booked_steps = (long long)c.stat[S_BOOKED];
+    stats->transport_steps[1] += stats->booked_steps;
     stats->bytes_per_track = (long long)sizeof(Rec<R>);
   }
   if (tout) tout->n = (int)std::min<long long>(c.extracted, INT32_MAX);

@@ -341,8 +341,9 @@ typedef struct {
   long long transport_read[3];    /* track records read */
   long long transport_written[3]; /* records written: survivors and interacting tracks */
   long long transport_queued[3];  /* of those, records written to the interaction buffers */
-  long long transport_steps[3];   /* steps completed in the transport kernel; e-: and the only steps of those that
-                              the interaction kernels book where they stop */
+  long long transport_steps[3];   /* steps completed in the transport kernel; e-: and booked_steps */
+  long long booked_steps;      /* steps of electrons that stop where they are created, booked by the
+                              interaction kernels and not made by the transport kernel of e- */
 } gx_transport_stats;
 
 void gx_transport_config_default(gx_transport_config *cfg);
