@@ -94,6 +94,9 @@ inline int default_blocks_per_sm(const gx_transport_config &c)
 // electrons in FP64 17.5, 16.9, 16.3; 20000 showers 131.5, 130.8, 129.6.  Fewer
 // steps of e- or e+ (1) or of photons (4) lost everywhere.
 constexpr int kDefaultSteps[3] = {16, 4, 2}, kFewSteps[3] = {6, 2, 2};
+// The same where the caller stops the run after a number of iterations: how far a
+// track comes in them is part of the result, so it depends on nothing else.
+constexpr int kCountedSteps[3] = {16, 16, 4};
 // Idle lanes of a warp before it takes new records in the transport kernel of
 // type q (0 gamma, 1 e-, 2 e+).  Measured: the FP32-mixed photon kernels of the
 // layered geometry gain 1.9% on C3, 2.7% on C4 and 0.9% with multiple

@@ -117,6 +117,7 @@ template <class R> struct Args {
   // the store has no more tracks than the grid has threads
   int step_budget[3], few_budget[3];
   int fetch_min[3];   // idle lanes of a warp before it takes new records, per particle type
+  int book_stops;     // electrons that stop where they are created may be booked there
 };
 
 // ---------------------------------------------------------------- geometry

@@ -402,10 +402,11 @@ template <class R, int PT, int K> __global__ void __launch_bounds__(1024, 1) k_t
 // them (n, the interactions of a launch) that throughput counts: 20000 showers
 // 128.9 to 123.7 ms, 256 events 169.8 to 163.7, 1001 through the volume tree 30.4
 // to 29.1, but two electrons 3.06 to 3.16, where the looking is latency on the way
-// to the next iteration.
-__device__ __forceinline__ bool local_stops(const Geom &g, long long n)
+// to the next iteration.  Not in a run whose caller counts its iterations (book_stops):
+// what is handed over after them would depend on n.
+template <class R> __device__ __forceinline__ bool local_stops(const Args<R> &a, long long n)
 {
-  return !g.msc && !g.charged_local && n >= 1024;
+  return a.book_stops && !a.g.msc && !a.g.charged_local && n >= 1024;
 }
 
 template <class R> __device__ __forceinline__ void book_stop(const Geom &g, const Track<R> &t, R e, Local &L)
@@ -514,7 +515,7 @@ __device__ __forceinline__ void interact_body(const Args<R> *__restrict__ A)
   Local L;
   tally_begin(L, a.g, a.edep, sm_edep, sm_stat, sm_esc, &sm_err);
 #ifndef GX_PARITY
-  const bool local = local_stops(a.g, n);
+  const bool local = local_stops(a, n);
 #endif
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long base = (long long)blockIdx.x * blockDim.x; base < n; base += stride) {
@@ -1249,14 +1250,17 @@ static int run(Ctx *C, const gx_transport_config *cfg, int nprim, const int *d_t
   }
   {
     // a budget asked for holds whatever the store's size; with
-    // steps_per_launch alone e+ get a quarter of it
+    // steps_per_launch alone e+ get a quarter of it.  A caller that counts
+    // iterations (max_iter) gets kCountedSteps, whatever the store's size, and no
+    // step beyond them.
+    L.a.book_stops = max_iter == 0;
     const int spl = cfg->steps_per_launch;
     for (int q = 0; q < 3; ++q) {
       const int asked = cfg->steps_per_launch_by_type[q] > 0 ? cfg->steps_per_launch_by_type[q]
                         : spl > 0                            ? (q == 2 ? std::max(1, spl / 4) : spl)
                                                              : 0;
-      L.a.step_budget[q] = asked ? asked : kDefaultSteps[q];
-      L.a.few_budget[q] = asked ? asked : kFewSteps[q];
+      L.a.step_budget[q] = asked ? asked : (max_iter > 0 ? kCountedSteps : kDefaultSteps)[q];
+      L.a.few_budget[q] = asked ? asked : (max_iter > 0 ? kCountedSteps : kFewSteps)[q];
     }
     // a warp refills when this many of its lanes are idle: a photon takes a
     // few cheap boundary-crossing steps, so the new-track work (record load,

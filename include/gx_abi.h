@@ -295,7 +295,9 @@ typedef struct {
                               at most (0: from capacity) */
   int steps_per_launch;    /* batched engine: steps of one track per transport launch, at most; a track
                               stays in registers between them (0: the engine's own choice, by particle type
-                              and by how many tracks there are; 1: one step per iteration) */
+                              and by how many tracks there are; 1: one step per iteration).  In runs to
+                              completion an electron that stops where it is created may take its only step
+                              in the iteration that creates it (booked_steps) */
   int msc;                 /* 1: multiple scattering of e-/e+ (Urban-type: safety-based step limit, true /
                               geometric path conversion, angular deflection); 2: the same with lateral
                               displacement (within the safety); 0: off (the reference has none,
@@ -535,7 +537,8 @@ int gx_post_step(gx_ctx *ctx, const gx_transport_config *cfg, gx_track_soa *trac
  * volume (< -1: located) -- and transported with their secondaries for at
  * most max_iterations iterations of the engine (0: to completion; one
  * iteration is one step of every track in flight with the plain engine,
- * up to steps_per_launch with the batched one), deposits added to d_edep.
+ * up to steps_per_launch with the batched one -- by default 16, e+ 4 -- however
+ * many tracks there are), deposits added to d_edep.
  * Every track still alive then -- in flight, deferred, or not yet injected --
  * is written to `out` (out->n set; status ALIVE), so a caller can hand tracks
  * over and take them back: transporting `out` afterwards, here or in the
