@@ -53,6 +53,20 @@ LAUNCH_KEYS = ("block_size", "blocks_per_sm", "steps_per_launch", "graph_iters",
 NSUB = 10  # sub-batches of a batch for the per-layer standard deviations
 
 
+def dominant_kernel(stats):
+    """The transport kernel with the most device time in a profiling run: particle
+    type, launches, ms, steps it made, records and bytes it read and wrote.  Steps are
+    without the e- steps that the interaction kernels book.  Bytes are the track
+    records (a track stays in registers from one step to the next, so they are fewer
+    than its steps): they do not bound the kernel, and no pipe does, but the latency
+    of its steps, dependent and divergent."""
+    k = int(np.argmax(stats["transport_ms"]))
+    steps = stats["transport_steps"][k] - (stats["booked_steps"] if k == 1 else 0)
+    records = stats["transport_read"][k] + stats["transport_written"][k]
+    return (k, max(1, stats["step_launches"][k]), stats["transport_ms"][k], steps, records,
+            records * stats["bytes_per_track"])
+
+
 def parse():
     p = argparse.ArgumentParser()
     p.add_argument("--gpus", type=int, default=1)
@@ -508,17 +522,7 @@ def main():
     # that takes the most device time (profiling pass, CUDA events around each
     # launch on the launching stream)
     stp = one(1, 1, profile=1)
-    k = int(np.argmax(stp["transport_ms"]))
-    launches_k = max(1, stp["step_launches"][k])
-    k_ms = stp["transport_ms"][k]
-    # the steps that the kernel makes: without the e- steps that the interaction kernels book
-    k_steps = stp["transport_steps"][k] - (stp["booked_steps"] if k == 1 else 0)
-    k_records = stp["transport_read"][k] + stp["transport_written"][k]
-    # algorithmic bytes: one read and one write of the track record per step
-    # (a step reads and writes the state once); the kernel keeps a track in
-    # registers across steps, so the records it actually moves are fewer
-    nbytes = k_steps * 2 * stp["bytes_per_track"]
-    moved = k_records * stp["bytes_per_track"]
+    k, launches_k, k_ms, k_steps, k_records, nbytes = dominant_kernel(stp)
     achieved = nbytes / (k_ms / 1e3) / 1e9
     peaks = {}
     try:
@@ -551,14 +555,12 @@ def main():
                 if len(f) >= 8:  # the same kernel on launches of the full batch
                     pipes["active_lanes_of_32_full_size"] = float(f[6])
                     pipes["issue_pct_full_size"] = float(f[7])
-    out["roofline"] = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                       "traffic": traffic,
+    out["roofline"] = {"bound": "latency", "against": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                       "frac": achieved / peak, "traffic": traffic,
                        "kernel": "k_transport<float,%d,0> (%s)" % (k, ["gamma", "e-", "e+"][k]),
                        "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
-                       "algorithmic_bytes_per_launch": nbytes / launches_k,
+                       "record_bytes_per_launch": nbytes / launches_k,
                        "steps_per_launch": k_steps / launches_k,
-                       "record_bytes_moved_per_launch": moved / launches_k,
-                       "record_bytes_moved_gbs": moved / (k_ms / 1e3) / 1e9,
                        "avg_launch_ms": k_ms / launches_k,
                        "share_of_step_kernel_time": k_ms / max(1e-9, sum(stp["step_ms"])),
                        "records_per_launch": k_records / launches_k,
