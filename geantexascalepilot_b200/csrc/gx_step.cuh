@@ -1,6 +1,7 @@
 // gx_step.cuh -- one step of a track, for the transport engine
-// (gx_transport.cu): the track record, the layered calorimeter's navigation, cross sections, multiple scattering, the phases of
-// a step, the interaction models' dispatch, and the tallies of a block.
+// (gx_transport.cu): the track record, the layered calorimeter's navigation, cross
+// sections, multiple scattering, the phases of a step, the interaction models'
+// dispatch, and the tallies of a block.
 #pragma once
 
 #include "gx_internal.cuh"
@@ -1349,15 +1350,13 @@ template <class R> struct RecWords {
   }
 };
 
-// L2: bypass L1 (the record may have been written on another SM since this one
-// last read its place)
-template <class R, bool L2 = false> __device__ __forceinline__ void load_rec(const Rec<R> *p, Track<R> &t)
+template <class R> __device__ __forceinline__ void load_rec(const Rec<R> *p, Track<R> &t)
 {
   RecWords<R> u;
   const uint4 *q = reinterpret_cast<const uint4 *>(p);
 #pragma unroll
   for (int k = 0; k < u.kWords / 4; ++k) {
-    const uint4 v = L2 ? __ldcg(&q[k]) : q[k];
+    const uint4 v = q[k];
     u.w[4 * k] = v.x;
     u.w[4 * k + 1] = v.y;
     u.w[4 * k + 2] = v.z;

@@ -1,17 +1,28 @@
-// gx_transport.cu -- the transport engine: every alive track takes one step
-// per iteration, in FP64 or FP32-mixed arithmetic.
+// gx_transport.cu -- the transport engine: every alive track takes one or more
+// steps per iteration, in FP64 or FP32-mixed arithmetic.
 //
 // Layout in HBM: per particle type (gamma, e-, e+) two track stores of
-// `capacity` records (current / next) and one overflow stack.  A step kernel
-// reads the current store of its type, runs one OneStep per track and writes
-// the survivor and its secondaries to the next stores through warp-aggregated
-// slot reservations (prefix sums over the warp, one atomic per warp and type),
-// so the stores stay compact and particle-pure without a separate compaction
-// pass.  Tracks that do not fit go to the stack and are re-injected when the
-// stores drain; primaries are injected on the device, with per-primary
+// `capacity` records (current / next), one overflow stack and a buffer for each
+// process.  A transport kernel reads the current store of its type and steps each
+// track, in registers, until it interacts (then it goes to the process's buffer),
+// ends, or has had its turn (then to the next store); an interaction kernel per
+// process reads its buffer and writes survivors and secondaries to the next
+// stores.  All are written at slots reserved per warp (ballots and one atomic for
+// each destination), so stores stay compact and particle-pure without a separate
+// compaction pass.  Tracks that do not fit go to the stack and are re-injected
+// when the stores drain; primaries are injected on the device, with per-primary
 // MRG32k3a substreams by skip-ahead, whenever fewer than `refill_below`
-// tracks are in flight.  The per-iteration launch sequence (refill, three
-// step kernels, finish) is captured once in a CUDA graph and replayed.
+// tracks are in flight.  The launches of an iteration (refill, three transport
+// kernels, eight interaction kernels on parallel branches, finish) are captured in
+// a CUDA graph that repeats on the device while tracks are left.
+//
+// Times in the comments of this file and of gx_step.cuh, gx_device.cuh and
+// gx_internal.cuh are ms per call on a B200 at 1965 MHz, with what is described and
+// without it, all else as it was at that time.  "20000 showers": 10^4 electrons and
+// 10^4 photons of 10 GeV, 50 layers, 4 T, FP32-mixed; "61 showers": 61 of them;
+// "256 events": 25600 electrons of 10 GeV from host arrays, scored in 256 events;
+// "two electrons": of 1 GeV, no field, FP64; "photons in lead": 10^4 of 10 MeV in a
+// lead cube, no field, FP64.
 //
 // The "plain" engine runs the same step code as one kernel over one mixed
 // store, launched and synchronised from the host every iteration, in FP64: the
@@ -165,7 +176,7 @@ template <class R, int K> constexpr int kMaxRegs = sizeof(R) == 8 ? 128 : (K == 
 // this file): per iteration and step kernel, the global timer when the first
 // block of the kernel starts and when the last one ends, so that a run shows
 // how the kernels of an iteration follow or overlap one another.  Kernel ids:
-// 0 refill, 1 refill bookkeeping, 2-4 transport of gamma, e-, e+, 5 + 3 type +
+// 0 refill, 1 refill bookkeeping (at a hand-over only), 2-4 transport of gamma, e-, e+, 5 + 3 type +
 // process the interaction kernels, 14 end of iteration; 512 iterations kept
 // (iteration i in row (i + 1) mod 512; row 0 holds the planning launch).
 // Without GX_TIMELINE the marks compile to nothing.
@@ -203,9 +214,9 @@ constexpr int kPhotonSteps = 4;
 // and steps it until the track interacts (it then goes to the interaction
 // buffer of its process), dies, leaves the world, or has taken step_budget
 // steps in this launch (it then goes to the next store).  A lane without a
-// track takes the next one of the current store from a work counter shared by
-// the whole grid (one atomic per warp for all its idle lanes), so the lanes
-// of a warp stay busy while their tracks take different numbers of steps.
+// track takes the next one of those that its warp has drawn, in chunks, from a
+// work counter shared by the whole grid, so the lanes of a warp stay busy while
+// their tracks take different numbers of steps.
 // One pass of the loop advances every lane by a few helix sub-steps (charged
 // tracks in a field), with the start and the end of a step attached to them, so
 // a lane whose step needs many sub-steps does not hold up the others.
@@ -223,10 +234,11 @@ template <class R, int PT, int K> __device__ __forceinline__ void transport_body
   const Store<R> &cur = a.st[par][PT];
   GX_TL_BEGIN(ctl, 2 + PT);
   const long long n = min(ctl->count[par][PT], cur.cap);
-  // Lanes of a warp that take records: one while the store has no more than one
-  // record per scheduler of the grid's SMs (a fifth of its warps), so that none
-  // waits for another's branches, else all (two electrons 3.87 against 3.47 ms;
-  // spread further, over all the warps, 61 showers lost 15%).
+  // Lanes of a warp that take records: one while the store has no more records than
+  // a fifth of the grid's warps (with 5 blocks of 128 threads per SM one for each
+  // scheduler, with 4 blocks 0.8), so that none waits for another's branches, else
+  // all (two electrons 3.87 against 3.47 ms; spread further, over all the warps, 61
+  // showers lost 15%).
   const int lanes = n <= (long long)gridDim.x * blockDim.x / 160 ? 1 : 32;
   if ((long long)blockIdx.x * (blockDim.x / 32) * lanes >= n) { // no work for this block (uniform exit)
     GX_TL_END();
@@ -255,9 +267,10 @@ template <class R, int PT, int K> __device__ __forceinline__ void transport_body
   unsigned read = 0, written = 0;
   // Records handed to this warp and not yet taken by a lane.  They come in
   // chunks of up to 32, one addition to the grid's counter per chunk instead of
-  // per pass, and on their way into L2 by the time a lane loads one: 20000
-  // showers 135.2 to 133.3 ms, 256 events 177.4 to 174.3.  A chunk is at most a
-  // quarter of a warp's share of the store, so that a small store is still spread
+  // per pass, and on their way into L2 by the time a lane loads one (a lane asks for
+  // the 128-byte line its record starts in; where a record ends in the next line,
+  // the next record starts there): 20000 showers 135.2 to 133.3 ms, 256 events 177.4
+  // to 174.3.  A chunk is at most a quarter of a warp's share of the store, so that a small store is still spread
   // over all warps (then 0: what is wanted, no more).
   long long pool_base = 0, old_base = 0;
   int pool_n = 0, old_n = 0;
@@ -395,15 +408,15 @@ template <class R, int PT, int K> __global__ void __launch_bounds__(1024, 1) k_t
 }
 
 #ifndef GX_PARITY
-// Electrons that stops_at_once() finds to end in the volume they are created in never become
-// records: about half of all e- steps are the only step of a photo-electron or a
-// Compton electron, and it leaves nothing but its deposit and its counts.
-// Without multiple scattering, and with enough of
-// them (n, the interactions of a launch) that throughput counts: 20000 showers
-// 128.9 to 123.7 ms, 256 events 169.8 to 163.7, 1001 through the volume tree 30.4
-// to 29.1, but two electrons 3.06 to 3.16, where the looking is latency on the way
-// to the next iteration.  Not in a run whose caller counts its iterations (book_stops):
-// what is handed over after them would depend on n.
+// Electrons that stops_at_once() finds to end in the volume they are created in
+// never become records: about half of all e- steps are the only step of a
+// photo-electron or a Compton electron, and it leaves nothing but its deposit and
+// its counts.  Without multiple scattering, and with enough of them (n, the
+// interactions of a launch) that throughput counts: 20000 showers 128.9 to 123.7
+// ms, 256 events 169.8 to 163.7, 1001 of 10 GeV through the volume tree 30.4 to
+// 29.1, but two electrons 3.06 to 3.16, where the looking is latency on the way to
+// the next iteration.  Not in a run whose caller counts its iterations
+// (book_stops): what is handed over after them would depend on n.
 template <class R> __device__ __forceinline__ bool local_stops(const Args<R> &a, long long n)
 {
   return a.book_stops && !a.g.msc && !a.g.charged_local && n >= 1024;
@@ -967,8 +980,6 @@ template <class R, int PT, int PROC> static void (*interact_for(const Launch<R> 
 {
 #ifndef GX_PARITY
   if (L.block > 256) return k_interact_wide<R, PT, PROC>;
-#endif
-#ifndef GX_PARITY
   if constexpr (PT == 0 && PROC != 1)
     if (L.a.g.geometry == 2)
       return sizeof(R) == 4 && L.a.g.csg.solids == kSolidsBox ? k_interact<R, PT, PROC, kSolidsBox>
@@ -980,7 +991,7 @@ template <class R, int PT, int PROC> static void (*interact_for(const Launch<R> 
 // One type's interaction kernels (gamma 3 processes, e- 2, e+ 3): one after
 // another, or (e given) the second and third on branches of their own beside
 // the first.  They read different buffers and reserve their outputs by atomics;
-// with few tracks each is 20 us of latency whatever its work: 61 showers 13.9 ms
+// with few tracks each is 10 to 20 us of latency whatever its work: 61 showers 13.9 ms
 // in a row, 12.5 side by side, two electrons 4.8 and 4.0, a full batch of 20000
 // 136.0 and 135.2.
 template <class R, int PT>
@@ -2225,9 +2236,6 @@ extern "C" int gx_transport_run_noalloc(gx_ctx *ctx, const gx_transport_config *
     if (hc.in_flight == 0 && hc.pending == 0) break;
     if (iters > 2000000LL) return set_error(GX_ERR_ITERCAP, "gx_transport_run_noalloc: iteration cap");
   }
-  if ((err = cudaMemcpyAsync(&hc, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-      (err = cudaStreamSynchronize(s)) != cudaSuccess)
-    return cuda_error(err, "gx_transport_run_noalloc: end");
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));
     stats->steps = (long long)hc.stat[S_STEPS];
